@@ -26,6 +26,12 @@ enum Field {
     F_PPU, F_PPV, F_PSI, F_SCG, NFIELDS
 };
 
+// Magnitudes of the D2V16 inverse moment matrix's entries (Ark/Lib/D2V16.cpp:14-52, names as
+// there): an entry is one of these times +-2^-k.
+struct D2V16Matrix {
+    double A, B, D, E, F, G, H, I, J, K, L, N, Pc, Qc, R, S, T, U, V, c23, ic, c12, jc;
+};
+
 // Constants of one case.  Names follow Ark/Constant/ZeroReference.h and
 // Ark/Constant/ZeroNamespace.h; all are derived on the host with the
 // reference's expressions (see host_params.cpp).
@@ -37,16 +43,18 @@ struct Params {
     double aTP, bTP, dtV;                          // 4/3, 1/3, dt/volume
     double T_CS, aCS;                              // Carnahan-Starling EOS
     // Reconstruction denominators as multipliers: -1/dx, -1/dy, 1/(2dy), 1/(-2dx).
-    // grad_mul = 1 when dx and dy are powers of two, so x/d == x*(1/d) exactly.
     double r_ndx, r_ndy, r_2dy, r_n2dx;
+    // divisors 6 2dx, 6 2dy, 6 MinL MinL, RT dt, and case constants scaled by a power of two
+    double g6x, g6y, lap6, RTdt, hDt2, dt2, Beta2, Kp2, NuV2, RT16, h_ah2;
+    double pp_ah2, pp_bh, pp_ch;  // pseudopotential face relaxation (half the first factor)
     // reciprocals RN(1/d) of divisors fixed per case, for the correctly rounded quotient
     // qdiv_rn: 1/RT, 1/(6 2dx), 1/(6 2dy), 1/(6 MinL MinL), 1/(W (PhiL - PhiV)), 1/(RT dt)
     double r_RT, r_g6x, r_g6y, r_lap, r_wI, r_RTdt;
-    int grad_mul, uw;                              // uw: upwind face reconstruction (DUGKS_FLUX_UW*)
+    int uw;                                        // uw: upwind face reconstruction (DUGKS_FLUX_UW*)
     int uw_grad;                                   // its cell gradient: 0 6-point, 1 least squares, 2 4-point
     double c16;                                    // D2V16 lattice speed
-    // D2V16 inverse moment matrix of this case, [16][16] in the case's device memory
-    // (Ark/Lib/D2V16.cpp:34-52): each case holds its own
+    D2V16Matrix m16;                               // its inverse moment matrix's magnitudes
+    // the matrix [16][16] in the case's device memory (Ark/Lib/D2V16.cpp:34-52; FMA variant)
     const double *iM16;
     double xi_u[16], xi_v[16], omega[16];
     int bb[16];
@@ -87,6 +95,14 @@ __host__ __device__ constexpr int d2q9_bb(int q) { return q == 0 ? 0 : (q <= 4 ?
 // not identically zero: the axis rings' rows (directions 0-3, 8-11) have none at the moments
 // 1, 2, 4, 13 and, for the directions along x, 8, 10, 11 (along y: 7, 9, 12).  Row q' of the
 // matrix holds row q's entries of the even moments and the negated entries of the odd ones.
+__host__ __device__ constexpr int d2v16_xu(int q) {
+    const int r = (q & 4) ? ((q & 3) == 0 || (q & 3) == 3 ? 1 : -1) : ((q & 3) == 0 ? 1 : ((q & 3) == 2 ? -1 : 0));
+    return q >= 8 ? 2 * r : r;
+}
+__host__ __device__ constexpr int d2v16_xv(int q) {
+    const int r = (q & 4) ? ((q & 3) <= 1 ? 1 : -1) : ((q & 3) == 1 ? 1 : ((q & 3) == 3 ? -1 : 0));
+    return q >= 8 ? 2 * r : r;
+}
 __host__ __device__ constexpr int d2v16_opp(int q) { return (q & ~3) | ((q + 2) & 3); }
 __host__ __device__ constexpr bool d2v16_odd_moment(int k) { return k == 1 || k == 2 || (k >= 7 && k <= 12); }
 __host__ __device__ constexpr bool d2v16_entry(int j, int k) {
@@ -95,7 +111,7 @@ __host__ __device__ constexpr bool d2v16_entry(int j, int k) {
                        ((j & 1) ? (k == 7 || k == 9 || k == 12) : (k == 8 || k == 10 || k == 11)));
 }
 
-// x * s for s in {-1, 0, 1}: exact, no multiply issued.
+// x * sign(s): exact, no multiply issued.
 __device__ __forceinline__ double sx(int s, double x) { return s > 0 ? x : (s < 0 ? -x : 0.0); }
 
 }  // namespace dugks

@@ -15,6 +15,53 @@
 
 namespace dugks {
 
+// Inverse moment matrix of the D2V16 model, from the closed-form
+// coefficients of Ark/Lib/D2V16.cpp:14-33 (c, e = (3+nK)c, nK = 0); the row
+// and column layout is the reference's (Ark/Lib/D2V16.cpp:34-52).
+static D2V16Matrix d2v16_magnitudes(double c) {
+    const double e = 3.0 * c;
+    const double c2 = c * c, e2 = e * e, c2e2 = c2 * e2;
+    const double A = 1.0 / (4.0 * e2), B = (-21.0 * c2 - e2) / (48.0 * c2e2), D = (7.0 * c2 + e2) / (32.0 * c2e2),
+                 E = (-3.0 * c2 - e2) / (96.0 * c2e2), F = 1.0 / (3.0 * c2),
+                 G = (3.0 * c2 - 5.0 * e2) / (4.0 * e2 * (e2 - 3.0 * c2)),
+                 H = 3.0 * (c2 + e2) / (4.0 * e2 * (e2 - 3.0 * c2)), I = (21.0 * c2 - 11.0 * e2) / (48.0 * c2e2),
+                 J = (21.0 * c2 * c2 - 32.0 * c2e2 + 11.0 * e2 * e2) / (32.0 * c2e2 * (e2 - 3.0 * c2)),
+                 K = (21.0 * c2 * c2 - 36.0 * c2e2 + 7.0 * e2 * e2) / (32.0 * c2e2 * (e2 - 3.0 * c2)),
+                 L = (3.0 * c2 - 5.0 * e2) / (96.0 * c2e2), N = 1.0 / (2.0 * c * e2),
+                 Pc = (3.0 * c2 - e2) / (12.0 * c2e2 * c), Qc = (c2 + e2) / (16.0 * c2e2 * c),
+                 R = (c2 - e2) / (16.0 * c2e2 * c), S = 1.0 / (24.0 * c2 * c2), T = 1.0 / (4.0 * c2 * (e2 - 3.0 * c2)),
+                 U = (c2 - e2) / (32.0 * c2 * c2 * (e2 - 3.0 * c2)),
+                 V = (5.0 * c2 - e2) / (32.0 * c2 * c2 * (e2 - 3.0 * c2));
+    return D2V16Matrix{A, B, D, E, F, G, H, I, J, K, L, N, Pc, Qc, R, S, T, U, V,
+                       2.0 / 3.0, 1.0 / (3.0 * c), 1.0 / 12, 1.0 / (24 * c)};
+}
+
+void build_d2v16_matrix(double c, double out[16][16]) {
+    const D2V16Matrix z = d2v16_magnitudes(c);
+    const double A = z.A, B = z.B, D = z.D, E = z.E, F = z.F, G = z.G, H = z.H, I = z.I, J = z.J, K = z.K, L = z.L,
+                 N = z.N, Pc = z.Pc, Qc = z.Qc, R = z.R, S = z.S, T = z.T, U = z.U, V = z.V, ic = z.ic, jc = z.jc;
+    // rows: ring 1 (axis c), ring 2 (diagonal c), ring 3 (axis 2c), ring 4 (diagonal 2c)
+    const double m[16][16] = {
+        {0, 0, 0, A, 0, G, H, N, 0, -N, 0, 0, -N, 0, T, -T},
+        {0, 0, 0, A, 0, H, G, 0, N, 0, -N, -N, 0, 0, -T, T},
+        {0, 0, 0, A, 0, G, H, -N, 0, N, 0, 0, N, 0, T, -T},
+        {0, 0, 0, A, 0, H, G, 0, -N, 0, N, N, 0, 0, -T, T},
+        {2.0 / 3.0, ic, ic, B, F, I, I, -N / 2, -N / 2, Pc, Pc, N / 2, N / 2, -S, S / 2, S / 2},
+        {2.0 / 3.0, -ic, ic, B, -F, I, I, N / 2, -N / 2, -Pc, Pc, N / 2, -N / 2, S, S / 2, S / 2},
+        {2.0 / 3.0, -ic, -ic, B, F, I, I, N / 2, N / 2, -Pc, -Pc, -N / 2, -N / 2, -S, S / 2, S / 2},
+        {2.0 / 3.0, ic, -ic, B, -F, I, I, -N / 2, N / 2, Pc, -Pc, -N / 2, N / 2, S, S / 2, S / 2},
+        {-0.5, 0, 0, D, 0, J, K, -N / 8, 0, Qc, 0, 0, R, 0, U, V},
+        {-0.5, 0, 0, D, 0, K, J, 0, -N / 8, 0, Qc, R, 0, 0, V, U},
+        {-0.5, 0, 0, D, 0, J, K, N / 8, 0, -Qc, 0, 0, -R, 0, U, V},
+        {-0.5, 0, 0, D, 0, K, J, 0, N / 8, 0, -Qc, -R, 0, 0, V, U},
+        {1.0 / 12, -jc, -jc, E, -F / 16, L, L, N / 16, N / 16, -Pc / 8, -Pc / 8, -R / 2, -R / 2, S / 4, S / 4, S / 4},
+        {1.0 / 12, jc, -jc, E, F / 16, L, L, -N / 16, N / 16, Pc / 8, -Pc / 8, -R / 2, R / 2, -S / 4, S / 4, S / 4},
+        {1.0 / 12, jc, jc, E, -F / 16, L, L, -N / 16, -N / 16, Pc / 8, Pc / 8, R / 2, R / 2, S / 4, S / 4, S / 4},
+        {1.0 / 12, -jc, jc, E, F / 16, L, L, N / 16, -N / 16, -Pc / 8, Pc / 8, R / 2, -R / 2, -S / 4, S / 4, S / 4}};
+    for (int a = 0; a < 16; ++a)
+        for (int b = 0; b < 16; ++b) out[a][b] = m[a][b];
+}
+
 void derive_params(const dugks_case_t &cs, const dugks_grid_t &g, Params &P) {
     P = Params{};
     P.nx = g.nx;
@@ -80,10 +127,7 @@ void derive_params(const dugks_case_t &cs, const dugks_grid_t &g, Params &P) {
         P.h_bh = 1.0 - P.h_ah;
         P.h_ch = tau * P.h_bh;
     }
-    {   // power-of-two spacings make every reconstruction division an exact multiply
-        int e;
-        const bool p2 = std::frexp(P.dx, &e) == 0.5 && std::frexp(P.dy, &e) == 0.5;
-        P.grad_mul = p2 ? 1 : 0;
+    {   // dx = dy = 1: every reconstruction division is an exact multiply
         P.r_ndx = 1.0 / (-P.dx);
         P.r_ndy = 1.0 / (-P.dy);
         P.r_2dy = 1.0 / (2 * P.dy);
@@ -97,6 +141,23 @@ void derive_params(const dugks_case_t &cs, const dugks_grid_t &g, Params &P) {
         P.r_lap = 1.0 / (6 * P.MinL * P.MinL);
         P.r_wI = 1.0 / (P.wI * (P.PhiL - P.PhiV));
         P.r_RTdt = 1.0 / (P.RT * P.dt);
+        P.g6x = P._2dx * 6;
+        P.g6y = P._2dy * 6;
+        P.lap6 = 6 * P.MinL * P.MinL;
+        P.RTdt = P.RT * P.dt;
+    }
+    {   // constants with a power of two taken in (exact)
+        P.hDt2 = 0.5 * P.hDt;
+        P.dt2 = 2 * P.dt;
+        P.Beta2 = 2 * P.Beta;
+        P.Kp2 = 0.5 * P.Kp;
+        P.NuV2 = 2 * P.NuV;
+        P.RT16 = P.RT / 16;
+        P.h_ah2 = 0.5 * P.h_ah;
+        const double tau = P.Tau0, ah = 2.0 * tau / (2.0 * tau + P.hDt);
+        P.pp_ah2 = 0.5 * ah;
+        P.pp_bh = 1.0 - ah;
+        P.pp_ch = tau * P.pp_bh;
     }
     P.uw = cs.flux_scheme != DUGKS_FLUX_CD ? 1 : 0;
     P.uw_grad = cs.flux_scheme == DUGKS_FLUX_UW_LS ? 1 : (cs.flux_scheme == DUGKS_FLUX_UW_4P ? 2 : 0);
@@ -112,6 +173,7 @@ void derive_params(const dugks_case_t &cs, const dugks_grid_t &g, Params &P) {
             P.omega[q] = 0.0;
             P.bb[q] = q;
         }
+        P.m16 = d2v16_magnitudes(MaSpan);
     } else {
         for (int q = 0; q < 9; ++q) {
             P.xi_u[q] = MaSpan * d2q9_xu(q);
@@ -120,46 +182,6 @@ void derive_params(const dugks_case_t &cs, const dugks_grid_t &g, Params &P) {
             P.bb[q] = d2q9_bb(q);
         }
     }
-}
-
-// Inverse moment matrix of the D2V16 model, from the closed-form
-// coefficients of Ark/Lib/D2V16.cpp:14-33 (c, e = (3+nK)c, nK = 0); the row
-// and column layout is the reference's (Ark/Lib/D2V16.cpp:34-52).
-void build_d2v16_matrix(double c, double out[16][16]) {
-    const double e = 3.0 * c;
-    const double c2 = c * c, e2 = e * e, c2e2 = c2 * e2;
-    const double A = 1.0 / (4.0 * e2), B = (-21.0 * c2 - e2) / (48.0 * c2e2), D = (7.0 * c2 + e2) / (32.0 * c2e2),
-                 E = (-3.0 * c2 - e2) / (96.0 * c2e2), F = 1.0 / (3.0 * c2),
-                 G = (3.0 * c2 - 5.0 * e2) / (4.0 * e2 * (e2 - 3.0 * c2)),
-                 H = 3.0 * (c2 + e2) / (4.0 * e2 * (e2 - 3.0 * c2)), I = (21.0 * c2 - 11.0 * e2) / (48.0 * c2e2),
-                 J = (21.0 * c2 * c2 - 32.0 * c2e2 + 11.0 * e2 * e2) / (32.0 * c2e2 * (e2 - 3.0 * c2)),
-                 K = (21.0 * c2 * c2 - 36.0 * c2e2 + 7.0 * e2 * e2) / (32.0 * c2e2 * (e2 - 3.0 * c2)),
-                 L = (3.0 * c2 - 5.0 * e2) / (96.0 * c2e2), N = 1.0 / (2.0 * c * e2),
-                 Pc = (3.0 * c2 - e2) / (12.0 * c2e2 * c), Qc = (c2 + e2) / (16.0 * c2e2 * c),
-                 R = (c2 - e2) / (16.0 * c2e2 * c), S = 1.0 / (24.0 * c2 * c2), T = 1.0 / (4.0 * c2 * (e2 - 3.0 * c2)),
-                 U = (c2 - e2) / (32.0 * c2 * c2 * (e2 - 3.0 * c2)),
-                 V = (5.0 * c2 - e2) / (32.0 * c2 * c2 * (e2 - 3.0 * c2));
-    // rows: ring 1 (axis c), ring 2 (diagonal c), ring 3 (axis 2c), ring 4 (diagonal 2c)
-    const double ic = 1.0 / (3.0 * c), jc = 1.0 / (24 * c);
-    const double m[16][16] = {
-        {0, 0, 0, A, 0, G, H, N, 0, -N, 0, 0, -N, 0, T, -T},
-        {0, 0, 0, A, 0, H, G, 0, N, 0, -N, -N, 0, 0, -T, T},
-        {0, 0, 0, A, 0, G, H, -N, 0, N, 0, 0, N, 0, T, -T},
-        {0, 0, 0, A, 0, H, G, 0, -N, 0, N, N, 0, 0, -T, T},
-        {2.0 / 3.0, ic, ic, B, F, I, I, -N / 2, -N / 2, Pc, Pc, N / 2, N / 2, -S, S / 2, S / 2},
-        {2.0 / 3.0, -ic, ic, B, -F, I, I, N / 2, -N / 2, -Pc, Pc, N / 2, -N / 2, S, S / 2, S / 2},
-        {2.0 / 3.0, -ic, -ic, B, F, I, I, N / 2, N / 2, -Pc, -Pc, -N / 2, -N / 2, -S, S / 2, S / 2},
-        {2.0 / 3.0, ic, -ic, B, -F, I, I, -N / 2, N / 2, Pc, -Pc, -N / 2, N / 2, S, S / 2, S / 2},
-        {-0.5, 0, 0, D, 0, J, K, -N / 8, 0, Qc, 0, 0, R, 0, U, V},
-        {-0.5, 0, 0, D, 0, K, J, 0, -N / 8, 0, Qc, R, 0, 0, V, U},
-        {-0.5, 0, 0, D, 0, J, K, N / 8, 0, -Qc, 0, 0, -R, 0, U, V},
-        {-0.5, 0, 0, D, 0, K, J, 0, N / 8, 0, -Qc, -R, 0, 0, V, U},
-        {1.0 / 12, -jc, -jc, E, -F / 16, L, L, N / 16, N / 16, -Pc / 8, -Pc / 8, -R / 2, -R / 2, S / 4, S / 4, S / 4},
-        {1.0 / 12, jc, -jc, E, F / 16, L, L, -N / 16, N / 16, Pc / 8, -Pc / 8, -R / 2, R / 2, -S / 4, S / 4, S / 4},
-        {1.0 / 12, jc, jc, E, -F / 16, L, L, -N / 16, -N / 16, Pc / 8, Pc / 8, R / 2, R / 2, S / 4, S / 4, S / 4},
-        {1.0 / 12, -jc, jc, E, F / 16, L, L, N / 16, -N / 16, -Pc / 8, Pc / 8, R / 2, -R / 2, -S / 4, S / 4, S / 4}};
-    for (int a = 0; a < 16; ++a)
-        for (int b = 0; b < 16; ++b) out[a][b] = m[a][b];
 }
 
 static void d2v16_eq_host(const Params &P, const double iM[16][16], double rho, double u, double v, double *eq) {
