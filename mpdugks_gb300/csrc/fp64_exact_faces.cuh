@@ -3,7 +3,7 @@
 // + Update_phi_h + Update_phiFlux_h (+ Wall_3_BB) -- Ark/Lib/D2Q9AC.cpp:106-144,
 // 232-329,345-358; Ark/Lib/D2Q9HCZ.cpp:93-131,183-271;
 // Ark/Cpp/DUGKS2DSolver.cpp:402-441; Ark/Cpp/Boundary.cpp:118-139.
-// UW: blockIdx.z 2 and 3 are the x and y periodic boundary faces in the
+// UW: the threads after the faces do the x and y periodic boundary faces in the
 // reference's low-side form (column 0 / row 0 only), written to xlo / ylo.
 // The x and y faces are separate bodies (XF), so each computes the six directions that cross
 // its face and no others.  The CD reconstruction gives twice the face values (b = SC times
@@ -122,12 +122,9 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
 
 template <int MODEL, bool WALLS, bool UW>
 __global__ void __launch_bounds__(256) k_faces_ac(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const bool xf = (blockIdx.z & 1) == 0;
-    const bool lo = UW && blockIdx.z >= 2;
-    const int nrows = xf ? P.ny : (WALLS ? P.ny + 1 : P.ny);
-    if (i >= P.nx || j >= nrows) return;
-    if (lo && (xf ? i != 0 : j != 0)) return;
+    int i, j;
+    bool xf, lo;
+    if (!face_of_thread(P, WALLS, UW, i, j, xf, lo)) return;
     if (xf) face_ac<MODEL, WALLS, UW, true>(P, S, i, j, lo);
     else face_ac<MODEL, WALLS, UW, false>(P, S, i, j, lo);
 }
@@ -209,9 +206,10 @@ __device__ __forceinline__ void face_pp1(const Params &P, const State &S, int i,
 }
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_faces_pp1(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
-    if (blockIdx.z == 0) face_pp1<MODEL, true>(P, S, i, j);
+    int i, j;
+    bool xf, lo;
+    if (!face_of_thread(P, false, false, i, j, xf, lo)) return;
+    if (xf) face_pp1<MODEL, true>(P, S, i, j);
     else face_pp1<MODEL, false>(P, S, i, j);
 }
 
@@ -253,9 +251,10 @@ __device__ __forceinline__ void face_pp2(const Params &P, const State &S, int i,
 }
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_faces_pp2(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
-    if (blockIdx.z == 0) face_pp2<MODEL, true>(P, S, i, j);
+    int i, j;
+    bool xf, lo;
+    if (!face_of_thread(P, false, false, i, j, xf, lo)) return;
+    if (xf) face_pp2<MODEL, true>(P, S, i, j);
     else face_pp2<MODEL, false>(P, S, i, j);
 }
 
@@ -265,8 +264,8 @@ __global__ void __launch_bounds__(256) k_faces_pp2(Params P, State S) {
 // Ark/Lib/D2Q9HCZ.cpp:133-182, Ark/Lib/D2Q9PP.cpp:89-109).
 template <int MODEL, bool WALLS>
 __global__ void __launch_bounds__(256) k_update(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
+    int i, j;
+    if (!cell_of_thread(P, i, j)) return;
     constexpr int Q = MODEL == PP16 ? 16 : 9;
     constexpr bool HASH = (MODEL == AC || MODEL == HCZ);
     const int pitch = P.pitch;

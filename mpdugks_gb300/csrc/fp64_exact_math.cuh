@@ -287,8 +287,8 @@ __device__ __forceinline__ double src_dot(int xu, int xv, double sx_, double sy_
 // (Ark/Cpp/PseudoP.cpp:31-38) first.
 template <int MODEL, bool WALLS>
 __global__ void __launch_bounds__(256) k_collide(Params P, State S, int do_msrc, int gin, int gout) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
+    int i, j;
+    if (!cell_of_thread(P, i, j)) return;
     const int pitch = P.pitch;
     const size_t c = (size_t)j * pitch + i;
     const double rho = S.fld[F_RHO][c], U = S.fld[F_U][c], V = S.fld[F_V][c], tau = S.fld[F_TAU][c];

@@ -3,7 +3,7 @@
 // + Update_phi_h + Update_phiFlux_h (+ Wall_3_BB) -- Ark/Lib/D2Q9AC.cpp:106-144,
 // 232-329,345-358; Ark/Lib/D2Q9HCZ.cpp:93-131,183-271;
 // Ark/Cpp/DUGKS2DSolver.cpp:402-441; Ark/Cpp/Boundary.cpp:118-139.
-// UW: blockIdx.z 2 and 3 are the x and y periodic boundary faces in the
+// UW: the threads after the faces do the x and y periodic boundary faces in the
 // reference's low-side form (column 0 / row 0 only), written to xlo / ylo.
 template <int MODEL, bool WALLS, bool UW, bool XF>
 __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, int j, bool lo, bool xrt) {
@@ -76,7 +76,7 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
         V = QDIV(sv, Rho * P.RT, inv);
         U += QDIV(0.5 * P.hDt * Fx, Rho * P.RT, inv);
         V += QDIV(0.5 * P.hDt * Fy, Rho * P.RT, inv);
-        p = sumf + 0.5 * P.hDt * P.RT * (Rho_x * U + Rho_y * V);
+        p = __fma_rn(0.5 * P.hDt * P.RT, Rho_x * U + Rho_y * V, sumf);
         Mu = P.NuV + (Phi - P.PhiV) * (P.NuL - P.NuV);
         Mu *= Rho;
         tauh = QDIV(Mu, Rho * P.RT, inv);
@@ -140,12 +140,9 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
 
 template <int MODEL, bool WALLS, bool UW>
 __global__ void __launch_bounds__(256) k_faces_ac(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const bool xf = (blockIdx.z & 1) == 0;
-    const bool lo = UW && blockIdx.z >= 2;
-    const int nrows = xf ? P.ny : (WALLS ? P.ny + 1 : P.ny);
-    if (i >= P.nx || j >= nrows) return;
-    if (lo && (xf ? i != 0 : j != 0)) return;
+    int i, j;
+    bool xf, lo;
+    if (!face_of_thread(P, WALLS, UW, i, j, xf, lo)) return;
     if (WALLS || xf) face_ac<MODEL, WALLS, UW, true>(P, S, i, j, lo, xf);
     else face_ac<MODEL, WALLS, UW, false>(P, S, i, j, lo, xf);
 }
@@ -154,9 +151,9 @@ __global__ void __launch_bounds__(256) k_faces_ac(Params P, State S) {
 // force, face pressure and psi (Ark/Lib/D2Q9PP.cpp:110-136, Ark/Cpp/PseudoP.cpp:23-30).
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_faces_pp1(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const bool xf = blockIdx.z == 0;
-    if (i >= P.nx || j >= P.ny) return;
+    int i, j;
+    bool xf, lo;
+    if (!face_of_thread(P, false, false, i, j, xf, lo)) return;
     constexpr int Q = MODEL == PP16 ? 16 : 9;
     const int im = wrapi(i - 1, P.nx), ip = wrapi(i + 1, P.nx);
     const size_t c = (size_t)j * P.pitch + i;
@@ -191,9 +188,9 @@ __global__ void __launch_bounds__(256) k_faces_pp1(Params P, State S) {
 // equilibrium, He-Shan-Doolen source and flux (Ark/Lib/D2Q9PP.cpp:97-105).
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_faces_pp2(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const bool xf = blockIdx.z == 0;
-    if (i >= P.nx || j >= P.ny) return;
+    int i, j;
+    bool xf, lo;
+    if (!face_of_thread(P, false, false, i, j, xf, lo)) return;
     constexpr int Q = MODEL == PP16 ? 16 : 9;
     const int nx = P.nx, ny = P.ny, pitch = P.pitch;
     const int im = wrapi(i - 1, nx), ip = wrapi(i + 1, nx), jm = wrapi(j - 1, ny), jp = wrapi(j + 1, ny);
@@ -231,8 +228,8 @@ __global__ void __launch_bounds__(256) k_faces_pp2(Params P, State S) {
 // Ark/Lib/D2Q9HCZ.cpp:133-182, Ark/Lib/D2Q9PP.cpp:89-109).
 template <int MODEL, bool WALLS>
 __global__ void __launch_bounds__(256) k_update(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
+    int i, j;
+    if (!cell_of_thread(P, i, j)) return;
     constexpr int Q = MODEL == PP16 ? 16 : 9;
     constexpr bool HASH = (MODEL == AC || MODEL == HCZ);
     const int pitch = P.pitch;

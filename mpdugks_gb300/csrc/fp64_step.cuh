@@ -81,6 +81,71 @@ __host__ __device__ constexpr int vel_u(int q) { return MODEL == PP16 ? d2v16_xu
 template <int MODEL>
 __host__ __device__ constexpr int vel_v(int q) { return MODEL == PP16 ? d2v16_xv(q) : d2q9_xv(q); }
 
+// Cells and faces of a launch.  Grids below BAND_THREADS threads: one-warp blocks whose threads
+// run over the cells in row order without regard to the rows' ends, so only the last warp has
+// idle lanes (a warp occupies the FP64 pipe alike however many lanes are active) and the
+// warps spread evenly over the SMs (a lone warp issues an FP64 instruction every 64 cycles,
+// an SM of four every 19: 256-thread blocks left most SMs of a small grid idle and others
+// with eight warps in turn).  Faces: the x-faces, then the y-faces (with walls one row
+// more), then (UW) the low-side x and y boundary faces, each group from a multiple of 32 on.
+// Larger grids have rounds of blocks enough for any shape, and 32 x 8 blocks (blockIdx.z: the
+// face group) read their y neighbours through L1 once: 2 % faster on 512x2048.
+// Passes of the benchmark's sizes, 32x8 blocks / one-warp blocks: 32x24 AC 2.67 / 1.86 ms, 128x128
+// AC 2.72 / 2.29, 256x256 D2V16 6.16 / 5.49, 333x257 HCZ (FMA) 9.49 / 8.16, 512x2048 HCZ 15.94 /
+// 16.27.
+constexpr unsigned BAND_THREADS = 32u * 152u * 100u;
+__device__ __forceinline__ bool cell_of_thread(const Params &P, int &i, int &j) {
+    if (blockDim.y > 1) {
+        i = blockIdx.x * 32 + threadIdx.x;
+        j = blockIdx.y * blockDim.y + threadIdx.y;
+        return i < P.nx && j < P.ny;
+    }
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    j = (int)(t / (unsigned)P.nx);
+    i = (int)(t - (unsigned)j * (unsigned)P.nx);
+    return j < P.ny;
+}
+__host__ __device__ __forceinline__ unsigned pad32(unsigned n) { return (n + 31u) & ~31u; }
+__device__ __forceinline__ bool face_of_thread(const Params &P, bool walls, bool uw, int &i, int &j, bool &xf, bool &lo) {
+    const unsigned nx = P.nx, ny = P.ny, yrows = walls ? ny + 1 : ny;
+    if (blockDim.y > 1) {
+        xf = (blockIdx.z & 1) == 0;
+        lo = uw && blockIdx.z >= 2;
+        i = blockIdx.x * 32 + threadIdx.x;
+        j = blockIdx.y * blockDim.y + threadIdx.y;
+        return (unsigned)i < nx && (unsigned)j < (xf ? ny : yrows) && !(lo && (xf ? i != 0 : j != 0));
+    }
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned nX = pad32(nx * ny), nY = pad32(nx * yrows);
+    lo = uw && t >= nX + nY;
+    if (lo) {
+        t -= nX + nY;
+        xf = t < pad32(ny);
+        if (!xf) t -= pad32(ny);
+        i = xf ? 0 : (int)t;
+        j = xf ? (int)t : 0;
+        return xf ? t < ny : t < nx;
+    }
+    xf = t < nX;
+    if (!xf) t -= nX;
+    j = (int)(t / nx);
+    i = (int)(t - (unsigned)j * nx);
+    return (unsigned)j < (xf ? ny : yrows);
+}
+struct Launch {
+    dim3 grid, block;
+};
+static Launch cell_launch(const Params &P) {
+    const unsigned nx = P.nx, ny = P.ny;
+    if (pad32(nx) * ny >= BAND_THREADS) return {dim3((nx + 31) / 32, (ny + 7) / 8), dim3(32, 8)};
+    return {dim3(pad32(nx * ny) / 32), dim3(32)};
+}
+static Launch face_launch(const Params &P, bool walls, bool uw) {
+    const unsigned nx = P.nx, ny = P.ny, yrows = walls ? ny + 1 : ny;
+    if (pad32(nx) * ny >= BAND_THREADS) return {dim3((nx + 31) / 32, (yrows + 7) / 8, uw ? 4 : 2), dim3(32, 8)};
+    return {dim3((pad32(nx * ny) + pad32(nx * yrows) + (uw ? pad32(ny) + pad32(nx) : 0)) / 32), dim3(32)};
+}
+
 // Cell field at logical row j in -1..ny (ghost rows: 2 a0 - a1 with walls,
 // wrap otherwise), column i already wrapped.
 template <bool WALLS>
@@ -110,8 +175,8 @@ __device__ __forceinline__ double cellv(const double *__restrict__ a, int ny, in
 // 6 _2dx, in the reference's operand order.
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_grad6(Params P, State S) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
+    int i, j;
+    if (!cell_of_thread(P, i, j)) return;
     const int pitch = P.pitch;
     const int im = wrapi(i - 1, P.nx), ip = wrapi(i + 1, P.nx), jm = wrapi(j - 1, P.ny), jp = wrapi(j + 1, P.ny);
     const size_t c = (size_t)j * pitch + i;
@@ -269,8 +334,8 @@ __global__ void __launch_bounds__(256) k_faces_nee(Params P, State S) {
 // handing the fields to the host).
 template <int MODEL, bool WALLS>
 __global__ void __launch_bounds__(256) k_finalize(Params P, State S, int gin) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
+    int i, j;
+    if (!cell_of_thread(P, i, j)) return;
     const size_t c = (size_t)j * P.pitch + i;
     if (MODEL == AC || MODEL == HCZ) {
         const double phi = S.fld[F_PHI][c], U = S.fld[F_U][c], V = S.fld[F_V][c];
@@ -363,20 +428,19 @@ __global__ void k_check_finite(const double *__restrict__ a, size_t n, int *flag
 template <int MODEL, bool WALLS>
 static void launch_step_t(const Params &P, const State &S, int do_msrc, int gin, int gout, cudaStream_t st,
                           int64_t *launches, cudaEvent_t *ev) {
-    const dim3 blk(32, 8);
-    const dim3 grd((P.nx + 31) / 32, (P.ny + 7) / 8);
+    const auto [grd, blk] = cell_launch(P);
     if (ev) cudaEventRecord(ev[0], st);
     k_collide<MODEL, WALLS><<<grd, blk, 0, st>>>(P, S, do_msrc, gin, gout);
     if (ev) cudaEventRecord(ev[1], st);
     if constexpr (MODEL == AC || MODEL == HCZ) {
         if (!WALLS && P.uw) {  // UW: cell gradients, then the faces with the low-side boundary faces
             k_grad6<MODEL><<<grd, blk, 0, st>>>(P, S);
-            const dim3 gf((P.nx + 31) / 32, (P.ny + 1 + 7) / 8, 4);
-            k_faces_ac<MODEL, false, true><<<gf, blk, 0, st>>>(P, S);
+            const auto [gf, bf] = face_launch(P, false, true);
+            k_faces_ac<MODEL, false, true><<<gf, bf, 0, st>>>(P, S);
             *launches += 4;
         } else {
-            const dim3 gf((P.nx + 31) / 32, (P.ny + 1 + 7) / 8, 2);
-            k_faces_ac<MODEL, WALLS, false><<<gf, blk, 0, st>>>(P, S);
+            const auto [gf, bf] = face_launch(P, WALLS, false);
+            k_faces_ac<MODEL, WALLS, false><<<gf, bf, 0, st>>>(P, S);
             *launches += 3;
             if (WALLS && P.nee) {  // NEE wall faces over the bounce-back ones
                 k_faces_nee<MODEL><<<dim3((P.nx + 127) / 128, 2), 128, 0, st>>>(P, S);
@@ -384,9 +448,9 @@ static void launch_step_t(const Params &P, const State &S, int do_msrc, int gin,
             }
         }
     } else {
-        const dim3 gf((P.nx + 31) / 32, (P.ny + 7) / 8, 2);
-        k_faces_pp1<MODEL><<<gf, blk, 0, st>>>(P, S);
-        k_faces_pp2<MODEL><<<gf, blk, 0, st>>>(P, S);
+        const auto [gf, bf] = face_launch(P, false, false);
+        k_faces_pp1<MODEL><<<gf, bf, 0, st>>>(P, S);
+        k_faces_pp2<MODEL><<<gf, bf, 0, st>>>(P, S);
         *launches += 4;
     }
     if (ev) cudaEventRecord(ev[2], st);
@@ -396,8 +460,7 @@ static void launch_step_t(const Params &P, const State &S, int do_msrc, int gin,
 
 template <int MODEL, bool WALLS>
 static void launch_finalize_t(const Params &P, const State &S, int gin, cudaStream_t st) {
-    const dim3 blk(32, 8);
-    const dim3 grd((P.nx + 31) / 32, (P.ny + 7) / 8);
+    const auto [grd, blk] = cell_launch(P);
     k_finalize<MODEL, WALLS><<<grd, blk, 0, st>>>(P, S, gin);
 }
 
