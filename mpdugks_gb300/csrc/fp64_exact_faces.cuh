@@ -9,29 +9,29 @@
 // its face and no others.  The CD reconstruction gives twice the face values (b = SC times
 // the stored number, SC = 1/2); the averaged source fields are kept as sums of the two cells
 // (twice the average) and their 1/2 goes into the constants they meet.
-template <int MODEL, bool WALLS, bool UW, bool XF>
+// EDGE: a face that reads the rows beyond a wall.
+template <int MODEL, bool EDGE, bool UW, bool XF>
 __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, int j, bool lo) {
-    const int nx = P.nx, ny = P.ny, pitch = P.pitch;
-    const int im = wrapi(i - 1, nx), ip = wrapi(i + 1, nx);
+    const int ny = P.ny, pitch = P.pitch;
     constexpr double SC = UW ? 1.0 : 0.5;
-    // owner/neighbour cells of this face and the summed source fields
-    int jo = XF ? j : j - 1;
-    const int io = XF ? im : i;
-    if (UW && jo < 0) jo += ny;  // periodic y (UW runs without walls)
+    const FaceRows r = face_rows(P, i, j);
+    // the source fields summed over the owner and the neighbour cell
     auto both = [&](int k) {
-        return cellv<WALLS>(S.fld[k], ny, pitch, jo, io) + cellv<WALLS>(S.fld[k], ny, pitch, j, i);
+        double o, n;
+        face_on<XF, EDGE>(P, S.fld[k], r, o, n);
+        return o + n;
     };
     double bf[9], bh[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
         const size_t qo = (size_t)q * S.qs;
         if (UW) {
-            const size_t co = (size_t)jo * pitch + io, cn = (size_t)j * pitch + i;
+            const size_t co = XF ? r.r0 + r.im : r.rm + i, cn = r.r0 + i;
             bf[q] = face_uw<XF>(P, S.bf + qo, S.gfx + qo, S.gfy + qo, co, cn, d2q9_xu(q), d2q9_xv(q), lo);
             bh[q] = face_uw<XF>(P, S.bh + qo, S.ghx + qo, S.ghy + qo, co, cn, d2q9_xu(q), d2q9_xv(q), lo);
         } else {
-            bf[q] = face_bh9<XF, WALLS>(P, S.bf + qo, i, im, ip, j, d2q9_xu(q), d2q9_xv(q));
-            bh[q] = face_bh9<XF, WALLS>(P, S.bh + qo, i, im, ip, j, d2q9_xu(q), d2q9_xv(q));
+            bf[q] = face_bh9<XF, EDGE>(P, S.bf + qo, r, d2q9_xu(q), d2q9_xv(q));
+            bh[q] = face_bh9<XF, EDGE>(P, S.bh + qo, r, d2q9_xu(q), d2q9_xv(q));
         }
     }
     double Phi = bh[0], sumf = bf[0];
@@ -104,7 +104,7 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
             hf = ahs * bf[q] + bh_ * (w * (m.p + m.rRT * G)) + ch * (0.5 * w * hcz_source(m, P.RT, G, xu, xv));
             hfo = ahs * bf[qo] + bh_ * (w * (m.p + m.rRT * Go)) + ch * (0.5 * w * hcz_source(m, P.RT, Go, -xu, -xv));
         }
-        if (WALLS && !XF) {  // bounce-back of the directions entering the fluid (xi.n_out < 0): q has xv > 0
+        if (EDGE && !XF) {  // bounce-back of the directions entering the fluid (xi.n_out < 0): q has xv > 0
             if (j == 0) {
                 hh = hho;
                 hf = hfo;
@@ -125,32 +125,36 @@ __global__ void __launch_bounds__(256) k_faces_ac(Params P, State S) {
     int i, j;
     bool xf, lo;
     if (!face_of_thread(P, WALLS, UW, i, j, xf, lo)) return;
-    if (xf) face_ac<MODEL, WALLS, UW, true>(P, S, i, j, lo);
-    else face_ac<MODEL, WALLS, UW, false>(P, S, i, j, lo);
+    if (WALLS && (j == 0 || (xf ? j == P.ny - 1 : j == P.ny))) {
+        if (xf) face_ac<MODEL, WALLS, UW, true>(P, S, i, j, lo);
+        else face_ac<MODEL, WALLS, UW, false>(P, S, i, j, lo);
+        return;
+    }
+    if (xf) face_ac<MODEL, false, UW, true>(P, S, i, j, lo);
+    else face_ac<MODEL, false, UW, false>(P, S, i, j, lo);
 }
 
 // Twice the half-step value of a D2V16 velocity xi = c (xu, xv), xu, xv in {-2 .. 2} known at
 // compile time: the products of the gradients with c once, the factors 2 and 1/4 exact.
 template <bool XF>
-__device__ __forceinline__ double face_bh16(const Params &P, const double *__restrict__ B, int i, int im, int ip,
-                                            int j, int xu, int xv) {
+__device__ __forceinline__ double face_bh16(const Params &P, const double *__restrict__ B, const FaceRows &r, int xu,
+                                            int xv) {
     double o, n;
-    face_on<XF, false>(P, B, i, im, j, o, n);
+    face_on<XF, false>(P, B, r, o, n);
     const double s = o + n;
     const int xn = XF ? xu : xv, xt = XF ? xv : xu;
     // g = (n - o) c xn + (t / 4) c xt; 2 hDt g = dt g, the factor of a ring (|xi| = c or 2 c) in dt
     const bool two = xn == 2 || xn == -2 || xt == 2 || xt == -2;
     const double k = two ? P.dt2 : P.dt;
     if (xt == 0) return s - k * sx(xn, (n - o) * P.c16);
-    const double t = face_tan<XF, false>(P, B, i, im, ip, j) * P.c16;
+    const double t = face_tan<XF, false>(P, B, r) * P.c16;
     if (xn == 0) return s - (two ? P.hDt : P.hDt2) * sx(xt, t);
     return s - k * __fma_rn(xt > 0 ? 0.25 : -0.25, t, sx(xn, (n - o) * P.c16));
 }
 template <int MODEL, bool XF>
-__device__ __forceinline__ double face_bhpp(const Params &P, const double *__restrict__ B, int i, int im, int ip,
-                                            int j, int q) {
-    return MODEL == PP16 ? face_bh16<XF>(P, B, i, im, ip, j, vel_u<MODEL>(q), vel_v<MODEL>(q))
-                         : face_bh9<XF, false>(P, B, i, im, ip, j, d2q9_xu(q), d2q9_xv(q));
+__device__ __forceinline__ double face_bhpp(const Params &P, const double *__restrict__ B, const FaceRows &r, int q) {
+    return MODEL == PP16 ? face_bh16<XF>(P, B, r, vel_u<MODEL>(q), vel_v<MODEL>(q))
+                         : face_bh9<XF, false>(P, B, r, d2q9_xu(q), d2q9_xv(q));
 }
 
 // first moments sum_q xi_q b_q over the directions with a nonzero component, the products
@@ -177,13 +181,13 @@ __device__ __forceinline__ void pp_first_moments(const Params &P, const double *
 template <int MODEL, bool XF>
 __device__ __forceinline__ void face_pp1(const Params &P, const State &S, int i, int j) {
     constexpr int Q = MODEL == PP16 ? 16 : 9;
-    const int im = wrapi(i - 1, P.nx), ip = wrapi(i + 1, P.nx);
-    const size_t c = (size_t)j * P.pitch + i;
+    const FaceRows r = face_rows(P, i, j);
+    const size_t c = r.r0 + i;
     double R, su, sv, b[Q];
     double *bo = XF ? S.xbf : S.ybf;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        b[q] = face_bhpp<MODEL, XF>(P, S.bf + (size_t)q * S.qs, i, im, ip, j, q);
+        b[q] = face_bhpp<MODEL, XF>(P, S.bf + (size_t)q * S.qs, r, q);
         bo[(size_t)q * S.qs + c] = b[q];
     }
     R = b[0];

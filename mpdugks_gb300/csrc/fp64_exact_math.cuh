@@ -421,23 +421,44 @@ __global__ void __launch_bounds__(256) k_collide(Params P, State S, int do_msrc,
 // The parts of one face and one velocity: s = o + n, the normal difference d = n - o along
 // +x / +y (XF: x-face between (im,j) and (i,j); else y-face between (i,j-1) and (i,j)), and
 // t, four times the tangential gradient along +y / +x.
-template <bool XF, bool WALLS>
-__device__ __forceinline__ void face_on(const Params &P, const double *__restrict__ B, int i, int im, int j, double &o,
-                                        double &n) {
-    o = XF ? cellv<WALLS>(B, P.ny, P.pitch, j, im) : cellv<WALLS>(B, P.ny, P.pitch, j - 1, i);
-    n = cellv<WALLS>(B, P.ny, P.pitch, j, i);
+// Cells around a face: offsets of the rows j - 1, j, j + 1 (wrapped); EDGE: a row beyond a wall
+// may be read, extrapolated by cellv (its 2 a0 - a1 at every load, predicated, made up a third
+// of the FP64 instructions when all rows went that way, so the other rows use offsets only).
+struct FaceRows {
+    int i, im, ip, j;
+    size_t rm, r0, rp;
+};
+__device__ __forceinline__ FaceRows face_rows(const Params &P, int i, int j) {
+    FaceRows r;
+    r.i = i;
+    r.im = wrapi(i - 1, P.nx);
+    r.ip = wrapi(i + 1, P.nx);
+    r.j = j;
+    r.rm = (size_t)wrapi(j - 1, P.ny) * P.pitch;
+    r.r0 = (size_t)wrapi(j, P.ny) * P.pitch;
+    r.rp = (size_t)wrapi(j + 1, P.ny) * P.pitch;
+    return r;
 }
-template <bool XF, bool WALLS>
-__device__ __forceinline__ double face_tan(const Params &P, const double *__restrict__ B, int i, int im, int ip,
-                                           int j) {
-    const int ny = P.ny, pitch = P.pitch;
+template <bool EDGE>
+__device__ __forceinline__ double at_row(const Params &P, const double *__restrict__ B, const FaceRows &r, int dj, int i) {
+    if (EDGE) return cellv<true>(B, P.ny, P.pitch, r.j + dj, i);
+    return B[(dj < 0 ? r.rm : (dj > 0 ? r.rp : r.r0)) + i];
+}
+template <bool XF, bool EDGE>
+__device__ __forceinline__ void face_on(const Params &P, const double *__restrict__ B, const FaceRows &r, double &o,
+                                        double &n) {
+    o = XF ? at_row<EDGE>(P, B, r, 0, r.im) : at_row<EDGE>(P, B, r, -1, r.i);
+    n = at_row<EDGE>(P, B, r, 0, r.i);
+}
+template <bool XF, bool EDGE>
+__device__ __forceinline__ double face_tan(const Params &P, const double *__restrict__ B, const FaceRows &r) {
     if (XF) {
-        const double SL = cellv<WALLS>(B, ny, pitch, j - 1, im), SR = cellv<WALLS>(B, ny, pitch, j - 1, i);
-        const double NL = cellv<WALLS>(B, ny, pitch, j + 1, im), NR = cellv<WALLS>(B, ny, pitch, j + 1, i);
+        const double SL = at_row<EDGE>(P, B, r, -1, r.im), SR = at_row<EDGE>(P, B, r, -1, r.i);
+        const double NL = at_row<EDGE>(P, B, r, 1, r.im), NR = at_row<EDGE>(P, B, r, 1, r.i);
         return (NR - SR) + (NL - SL);
     }
-    const double WB = cellv<WALLS>(B, ny, pitch, j - 1, im), EB = cellv<WALLS>(B, ny, pitch, j - 1, ip);
-    const double WT = cellv<WALLS>(B, ny, pitch, j, im), ET = cellv<WALLS>(B, ny, pitch, j, ip);
+    const double WB = at_row<EDGE>(P, B, r, -1, r.im), EB = at_row<EDGE>(P, B, r, -1, r.ip);
+    const double WT = at_row<EDGE>(P, B, r, 0, r.im), ET = at_row<EDGE>(P, B, r, 0, r.ip);
     return (ET - WT) + (EB - WB);
 }
 // Twice the half-step value of a D2Q9 velocity xi = (xu, xv), components in {-1, 0, 1} known
@@ -446,16 +467,16 @@ __device__ __forceinline__ double face_tan(const Params &P, const double *__rest
 // and its sum with the other term only decide the sign of a zero result).  1, 3, 5 and 7
 // FP64 operations for the rest, the normal, the tangential and the diagonal directions
 // (the value itself, with every factor applied: 2, 6, 9 and 12).
-template <bool XF, bool WALLS>
-__device__ __forceinline__ double face_bh9(const Params &P, const double *__restrict__ B, int i, int im, int ip,
-                                           int j, int xu, int xv) {
+template <bool XF, bool EDGE>
+__device__ __forceinline__ double face_bh9(const Params &P, const double *__restrict__ B, const FaceRows &r, int xu,
+                                           int xv) {
     double o, n;
-    face_on<XF, WALLS>(P, B, i, im, j, o, n);
+    face_on<XF, EDGE>(P, B, r, o, n);
     const double s = o + n;
     const int xn = XF ? xu : xv, xt = XF ? xv : xu;
     if (xn == 0 && xt == 0) return s;
     if (xt == 0) return __fma_rn(xn > 0 ? -0.5 : 0.5, n - o, s);
-    const double t = face_tan<XF, WALLS>(P, B, i, im, ip, j);
+    const double t = face_tan<XF, EDGE>(P, B, r);
     if (xn == 0) return __fma_rn(xt > 0 ? -0.125 : 0.125, t, s);
     const double g = __fma_rn(xt > 0 ? 0.25 : -0.25, t, xn > 0 ? n - o : o - n);
     return __fma_rn(-0.5, g, s);
