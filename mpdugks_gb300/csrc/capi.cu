@@ -177,23 +177,15 @@ template <typename R>
 static void derive_p32(const Params &P, f32::PR<R> &Q) {
     Q = f32::PR<R>{};
     Q.nx = P.nx; Q.ny = P.ny; Q.pitch = P.pitch; Q.walls = P.walls; Q.model = P.model; Q.gravity = P.gravity;
-    Q.phi0 = (R)DUGKS_F32_PHI0; Q.p0 = R(1.0);
-    Q.aPhi = (R)P.aPhi; Q.bPhi = (R)P.bPhi; Q.Kp = (R)P.Kp; Q.RT = (R)P.RT;
-    Q.invRT = (R)(1.0 / P.RT); Q.hDt = (R)P.hDt; Q.dt = (R)P.dt; Q.Lambda0 = (R)P.Lambda0;
-    Q.Beta = (R)P.Beta; Q.Kappa = (R)P.Kappa; Q.PhiL = (R)P.PhiL; Q.PhiV = (R)P.PhiV;
+    Q.aPhi = (R)P.aPhi; Q.bPhi = (R)P.bPhi; Q.Beta = (R)P.Beta; Q.Kappa = (R)P.Kappa;
     Q.RhoL = (R)P.RhoL; Q.Gy = (R)P.Gy;
-    Q.inv_12dx = (R)(1.0 / (P._2dx * 6)); Q.inv_12dy = (R)(1.0 / (P._2dy * 6));
-    Q.inv_6dd = (R)(1.0 / (6 * P.MinL * P.MinL));
     Q.inv_wI_dphi = (R)(1.0 / (P.wI * (P.PhiL - P.PhiV)));
-    Q.inv_RTdt = (R)(1.0 / (P.RT * P.dt));
     // after the first step tau = Mu/(rho RT) = Tau0 for both Allen-Cahn models (nu_L = nu_V = nu0)
     const double tau = P.Tau0;
     const double aBP = (2.0 * tau - P.hDt) / (2.0 * tau + P.dt), ah = 2.0 * tau / (2.0 * tau + P.hDt);
     Q.tauf = (R)tau; Q.aBP_f = (R)aBP; Q.ah_f = (R)ah;
     Q.h_aBP = (R)P.h_aBP; Q.h_bBP = (R)P.h_bBP; Q.h_cBP = (R)P.h_cBP;
     Q.h_ah = (R)P.h_ah; Q.h_bh = (R)P.h_bh; Q.h_ch = (R)P.h_ch;
-    Q.r_2dy = (R)P.r_2dy; Q.r_ndx = (R)P.r_ndx; Q.r_n2dx = (R)P.r_n2dx; Q.r_ndy = (R)P.r_ndy;
-    Q.aTP = (R)P.aTP; Q.bTP = (R)P.bTP; Q.dtV = (R)P.dtV;
     Q.nee = P.nee;
     Q.uw_grad = P.uw_grad;
     Q.hneq = (R)(2.0 * P.TauMass / (2.0 * P.TauMass + P.dt));

@@ -12,6 +12,15 @@
 namespace dugks {
 namespace f32 {
 
+// Every sum of two products here names the product that is rounded (mulr) and the one that is
+// fused: a compiler left to contract chooses by the uses of a product, so the same formula
+// rounds differently in two kernels, and differently again when a constant folds -- and the
+// velocity of a nearly resting fluid shows it at 1e-5 of its norm.
+__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mulr(double a, double b) { return __dmul_rn(a, b); }
+// a b + c d, the first product fused, the second rounded
+template <typename R>
+__device__ __forceinline__ R mad2(R a, R b, R c, R d) { return fma(a, b, mulr(c, d)); }
 template <typename R>
 __device__ __forceinline__ R sxf(int s, R x) { return s > 0 ? x : (s < 0 ? -x : R(0)); }
 
@@ -55,12 +64,12 @@ __device__ __forceinline__ V ff_sum9(const V (&a)[9]) {
 template <int MODEL, typename R>
 __device__ __forceinline__ void cell_macros(const PR<R> &P, const R *df, R phi, R fx_old, R fy_old, R rx_old,
                                             R ry_old, R &rho, R &U, R &V, R &dp) {
-    rho = P.aPhi * phi + P.bPhi;
+    rho = fma(P.aPhi, phi, P.bPhi);
     if (MODEL == AC) {
         const R fa[9] = {R(0.), df[1], df[2], df[3], df[4], df[5], df[6], df[7], df[8]};
         U = R(0.);
         V = R(0.);
-        dp = ff_sum9(fa) * P.Kp;
+        dp = mulr(ff_sum9(fa), P.Kp);
     } else {
         R ua[9], va[9], fa[9];
 #pragma unroll
@@ -70,10 +79,10 @@ __device__ __forceinline__ void cell_macros(const PR<R> &P, const R *df, R phi, 
             va[q] = sxf(d2q9_xv(q), df[q]);
         }
         const R su = ff_sum9(ua), sv = ff_sum9(va), sfv = ff_sum9(fa);
-        const R inv = R(1.) / (rho * P.RT);
-        U = su * inv + P.hDt * fx_old * inv;
-        V = sv * inv + P.hDt * fy_old * inv;
-        dp = sfv + P.hDt * (rx_old * U + ry_old * V) * P.RT;
+        const R inv = R(1.) / mulr(rho, P.RT);
+        U = mad2(su, inv, P.hDt * fx_old, inv);
+        V = mad2(sv, inv, P.hDt * fy_old, inv);
+        dp = fma(P.hDt * mad2(rx_old, U, ry_old, V), P.RT, sfv);
     }
 }
 
@@ -93,27 +102,27 @@ __device__ __forceinline__ void macro_source9(const PR<R> &P, R phi, T C, const 
     for (int k = 0; k < 8; ++k) d[k] = (ph[k].x - C.x) + (ph[k].y - C.y);
     const R E = d[0], W = d[1], N = d[2], S = d[3], NE = d[4], NW = d[5], SE = d[6], SW = d[7];
     // mirror-symmetric association: x -> -x maps every sum onto its exact negation
-    R gx = (R(4.) * (E - W) + ((NE - NW) + (SE - SW))) * P.inv_12dx;
-    R gy = (R(4.) * (N - S) + ((NE - SE) + (NW - SW))) * P.inv_12dy;
-    const R lap = (R(4.) * ((E + W) + (N + S)) + ((NE + SW) + (NW + SE))) * P.inv_6dd;
+    R gx = mulr(fma(R(4.), E - W, (NE - NW) + (SE - SW)), P.inv_12dx);
+    R gy = mulr(fma(R(4.), N - S, (NE - SE) + (NW - SW)), P.inv_12dy);
+    const R lap = mulr(fma(R(4.), (E + W) + (N + S), (NE + SW) + (NW + SE)), P.inv_6dd);
     if (fabs(gx) < R(DUGKS_F32_GCLAMP)) gx = R(0.);
     if (fabs(gy) < R(DUGKS_F32_GCLAMP)) gy = R(0.);
-    const R F = R(2.) * P.Beta * (phi - P.PhiL) * (phi - P.PhiV) * (R(2.) * phi - P.PhiL - P.PhiV) - P.Kappa * lap;
-    rhox = P.aPhi * gx;
-    rhoy = P.aPhi * gy;
-    fx = F * gx;
-    fy = F * gy;
-    if (P.gravity) fy -= P.Gy * (rho - P.RhoL);
-    const R L2 = gx * gx + gy * gy;
-    const R dU = phi * U - ppu, dV = phi * V - ppv;
+    const R F = mad2(mulr(mulr(mulr(R(2.), P.Beta), phi - P.PhiL), phi - P.PhiV), fma(R(2.), phi, -P.PhiL) - P.PhiV, -P.Kappa, lap);
+    rhox = mulr(P.aPhi, gx);
+    rhoy = mulr(P.aPhi, gy);
+    fx = mulr(F, gx);
+    fy = mulr(F, gy);
+    if (P.gravity) fy = fma(-P.Gy, rho - P.RhoL, fy);
+    const R L2 = mad2(gx, gx, gy, gy);
+    const R dU = fma(phi, U, -ppu), dV = fma(phi, V, -ppv);
     if (L2 != R(0.)) {
-        const R tmp = -R(4.) * (phi - P.PhiL) * (phi - P.PhiV) * P.inv_wI_dphi;
-        const R k = tmp * rsq(L2);
-        srcx = gx * k + dU * P.inv_RTdt;
-        srcy = gy * k + dV * P.inv_RTdt;
+        const R tmp = mulr(mulr(mulr(-R(4.), phi - P.PhiL), phi - P.PhiV), P.inv_wI_dphi);
+        const R k = mulr(tmp, rsq(L2));
+        srcx = mad2(dU, P.inv_RTdt, gx, k);
+        srcy = mad2(dV, P.inv_RTdt, gy, k);
     } else {
-        srcx = dU * P.inv_RTdt;
-        srcy = dV * P.inv_RTdt;
+        srcx = mulr(dU, P.inv_RTdt);
+        srcy = mulr(dV, P.inv_RTdt);
     }
 }
 
@@ -229,7 +238,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 template <typename R>
 struct EqSite {
     typename Pair<R>::T A2, D2;
-    R Ux, Vx, uuL, UF, UR, fx, fy, rx, ry, sx, sy, fxI, fyI, dpI;
+    R U, V, Ux, Vx, uu, UF, UR, fx, fy, rx, ry, sx, sy, fxI, fyI, dpI;
 };
 template <int MODEL, typename R>
 __device__ __forceinline__ EqSite<R> eq_site(const PR<R> &P, R U, R V, R uu, R rho, R phi, R dp, R dphi, R fx,
@@ -240,22 +249,34 @@ __device__ __forceinline__ EqSite<R> eq_site(const PR<R> &P, R U, R V, R uu, R r
     e.sx = sx_;
     e.sy = sy_;
     if (MODEL == AC) {
-        e.fxI = fx * P.invRT;
-        e.fyI = fy * P.invRT;
-        e.dpI = dp * P.invRT;
+        e.fxI = mulr(fx, P.invRT);
+        e.fyI = mulr(fy, P.invRT);
+        e.dpI = mulr(dp, P.invRT);
         e.D2 = mk2(e.dpI, dphi);
     } else {
-        e.Ux = U * P.invRT;
-        e.Vx = V * P.invRT;
-        e.uuL = uu * P.Lambda0;
-        e.UF = U * fx + V * fy;
-        e.UR = U * rx + V * ry;
+        e.U = U;
+        e.V = V;
+        e.Ux = mulr(U, P.invRT);
+        e.Vx = mulr(V, P.invRT);
+        e.uu = uu;
+        e.UF = mad2(U, fx, V, fy);
+        e.UR = mad2(U, rx, V, ry);
         e.rx = rx;
         e.ry = ry;
-        e.A2 = mk2(rho * P.RT, phi);
+        e.A2 = mk2(mulr(rho, P.RT), phi);
         e.D2 = mk2(dp, dphi);
     }
     return e;
+}
+
+// (xi_Q.a) / RT for Q in {1, 2, 3, 4}, from a = (x, y) and its quotients xI, yI: on the diagonals
+// one of the two quotients is fused into the sum, y's at an x-face (XF), else x's
+template <int Q, bool XF, typename R>
+__device__ __forceinline__ R xi_over_RT(const PR<R> &P, R x, R xI, R y, R yI) {
+    if (Q == 1) return xI;
+    if (Q == 3) return yI;
+    if (XF) return fma(y, P.invRT, Q == 2 ? xI : -xI);
+    return fma(Q == 2 ? x : -x, P.invRT, yI);
 }
 
 // Equilibrium deviations and force terms, as (f, h) pairs, of direction Q in
@@ -264,32 +285,32 @@ __device__ __forceinline__ EqSite<R> eq_site(const PR<R> &P, R U, R V, R uu, R r
 //   So = (w (A + G (A + RT B)), w xi.src) with A = xi.F - u.F, B = xi.grad rho -
 //   u.grad rho, G = u1 + u1^2/2 - |u|^2 lambda (= (1+G)(c.F) + G RT (c.grad rho),
 //   c = xi - u), u1 = xi.u / RT.
-template <int MODEL, int Q, typename R>
+template <int MODEL, int Q, bool XF, typename R>
 __device__ __forceinline__ void eq_pair(const PR<R> &P, const EqSite<R> &e, typename Pair<R>::T &Eq,
                                         typename Pair<R>::T &So, typename Pair<R>::T &Eqb,
                                         typename Pair<R>::T &Sob) {
     constexpr int xu = d2q9_xu(Q), xv = d2q9_xv(Q);
     const R wq = (R)d2q9_w(Q);
-    const R hS = wq * (sxf(xu, e.sx) + sxf(xv, e.sy));
+    const R hS = mulr(wq, sxf(xu, e.sx) + sxf(xv, e.sy));
     if (MODEL == AC) {
         Eq = mul2(mk2(wq, wq), e.D2);
         Eqb = Eq;
-        const R sf = wq * (sxf(xu, e.fxI) + sxf(xv, e.fyI));
+        const R sf = mulr(wq, xi_over_RT<Q, XF>(P, e.fx, e.fxI, e.fy, e.fyI));
         So = mk2(sf, hS);
         Sob = mk2(-sf, -hS);
     } else {
-        const R u1 = sxf(xu, e.Ux) + sxf(xv, e.Vx);
-        const R H = (R(0.5) * u1) * u1 - e.uuL;
+        const R u1 = xi_over_RT<Q, XF>(P, e.U, e.Ux, e.V, e.Vx);
+        const R H = mad2(R(0.5) * u1, u1, -e.uu, P.Lambda0);
         const R G = H + u1, Gb = H - u1;
         const R eF = sxf(xu, e.fx) + sxf(xv, e.fy), eR = sxf(xu, e.rx) + sxf(xv, e.ry);
         const R A = eF - e.UF, Ab = -eF - e.UF;
         const R B = eR - e.UR, Bb = -eR - e.UR;
-        const R C = P.RT * B + A, Cb = P.RT * Bb + Ab;
+        const R C = fma(P.RT, B, A), Cb = fma(P.RT, Bb, Ab);
         const auto w2 = mk2(wq, wq);
         Eq = mul2(w2, fma2(e.A2, mk2(G, u1), e.D2));
         Eqb = mul2(w2, fma2(e.A2, mk2(Gb, -u1), e.D2));
-        So = mk2(wq * (G * C + A), hS);
-        Sob = mk2(wq * (Gb * Cb + Ab), -hS);
+        So = mk2(mulr(wq, fma(G, C, A)), hS);
+        Sob = mk2(mulr(wq, fma(Gb, Cb, Ab)), -hS);
     }
 }
 
@@ -339,10 +360,10 @@ __device__ __forceinline__ void collide_cell(const PR<R> &P, const SR<R> &S, lon
         aBP = (R(2.) * tau - P.hDt) / (R(2.) * tau + P.dt);
         cBP = tau * (R(1.) - aBP);
     } else {
-        rho = P.aPhi * phi + P.bPhi;
+        rho = fma(P.aPhi, phi, P.bPhi);
         R ppu = R(0.), ppv = R(0.);
         if (MODEL == AC) {
-            dp = sfz * P.Kp;
+            dp = mulr(sfz, P.Kp);
         } else {
             const R fxo = a6[A_FX], fyo = a6[A_FY];
             rxo = a6[A_RHOX];
@@ -354,25 +375,25 @@ __device__ __forceinline__ void collide_cell(const PR<R> &P, const SR<R> &S, lon
                              mk2(R(0.), Pq[3].x),   mk2(-Pq[4].x, Pq[4].x), mk2(-Pq[5].x, R(0.)),
                              mk2(-Pq[6].x, -Pq[6].x), mk2(R(0.), -Pq[7].x), mk2(Pq[8].x, -Pq[8].x)};
             const T mv = dev_sum9(mt);
-            const R inv = rcp(rho * P.RT);
-            U = mv.x * inv + P.hDt * fxo * inv;
-            V = mv.y * inv + P.hDt * fyo * inv;
-            dp = sfz + P.hDt * (rxo * U + ryo * V) * P.RT;
+            const R inv = rcp(mulr(rho, P.RT));
+            U = mad2(P.hDt * fxo, inv, mv.x, inv);
+            V = mad2(P.hDt * fyo, inv, mv.y, inv);
+            dp = fma(P.hDt * mad2(rxo, U, ryo, V), P.RT, sfz);
         }
         macro_source9(P, phi, pc, ph, rho, U, V, ppu, ppv, srcx, srcy, rhox, rhoy, fx, fy);
         aBP = P.aBP_f;  // tau is constant after the first step (nu_L = nu_V)
-        cBP = P.tauf * (R(1.) - aBP);
+        cBP = mulr(P.tauf, R(1.) - aBP);
     }
     const R bBP = R(1.) - aBP;
-    const R uu = U * U + V * V;
+    const R uu = mad2(U, U, V, V);
     // equilibria of q != 0; q = 0 from the exact zeroth moment (sum dEq = dp for
     // HCZ, 0 for AC; sum (h_eq - w phi) = 0), so FP32 weights cannot leak mass
     T Eq[9], So[9];
     const EqSite<R> es = eq_site<MODEL, R>(P, U, V, uu, rho, phi, dp, R(0.), fx, fy, rhox, rhoy, srcx, srcy);
-    eq_pair<MODEL, 1>(P, es, Eq[1], So[1], Eq[5], So[5]);
-    eq_pair<MODEL, 2>(P, es, Eq[2], So[2], Eq[6], So[6]);
-    eq_pair<MODEL, 3>(P, es, Eq[3], So[3], Eq[7], So[7]);
-    eq_pair<MODEL, 4>(P, es, Eq[4], So[4], Eq[8], So[8]);
+    eq_pair<MODEL, 1, false>(P, es, Eq[1], So[1], Eq[5], So[5]);
+    eq_pair<MODEL, 2, false>(P, es, Eq[2], So[2], Eq[6], So[6]);
+    eq_pair<MODEL, 3, false>(P, es, Eq[3], So[3], Eq[7], So[7]);
+    eq_pair<MODEL, 4, false>(P, es, Eq[4], So[4], Eq[8], So[8]);
     const T sEq = sym8p(Eq);
     Eq[0] = sub2(mk2(MODEL == AC ? R(0.) : dp, R(0.)), sEq);
     if (MODEL == AC) {
@@ -391,7 +412,7 @@ __device__ __forceinline__ void collide_cell(const PR<R> &P, const SR<R> &S, lon
     // phase field sum_q h is conserved (sum Eq = phi, sum S = 0); HCZ flow
     //   (1-a)(p - sum f) + c sum S = (1-a) hDt RT (grad rho_old . u) + c RT (u . grad rho)
     const T sInc = sym8p(inc);
-    const R z0 = MODEL == HCZ ? (bBP * P.hDt * P.RT * (rxo * U + ryo * V) + cBP * P.RT * (U * rhox + V * rhoy)) - sInc.x
+    const R z0 = MODEL == HCZ ? mad2(mulr(bBP * P.hDt, P.RT), mad2(rxo, U, ryo, V), mulr(cBP, P.RT), es.UR) - sInc.x
                               : inc[0].x;
     inc[0] = mk2(z0, -sInc.y);
     src[0] = srcx;
@@ -545,20 +566,20 @@ __device__ __forceinline__ void face_state_flux(const PR<R> &P, const typename P
     const R su = (bh[1].x - bh[5].x) + ((bh[2].x - bh[6].x) + (bh[8].x - bh[4].x));
     const R sv = (bh[3].x - bh[7].x) + ((bh[2].x - bh[6].x) + (bh[4].x - bh[8].x));
     const R phif = avg + dphif;
-    const R rhof = P.aPhi * phif + P.bPhi;
+    const R rhof = fma(P.aPhi, phif, P.bPhi);
     R Uf, Vf, dpf;
     if (MODEL == AC) {
         Uf = R(0.);
         Vf = R(0.);
-        dpf = sf * P.Kp;
+        dpf = mulr(sf, P.Kp);
     } else {
-        const R inv = rcp(rhof * P.RT);
-        Uf = su * inv + R(0.5) * P.hDt * av[4] * inv;
-        Vf = sv * inv + R(0.5) * P.hDt * av[5] * inv;
-        dpf = sf + R(0.5) * P.hDt * P.RT * (av[2] * Uf + av[3] * Vf);
+        const R inv = rcp(mulr(rhof, P.RT));
+        Uf = mad2(su, inv, R(0.5) * P.hDt * av[4], inv);
+        Vf = mad2(sv, inv, R(0.5) * P.hDt * av[5], inv);
+        dpf = fma(R(0.5) * P.hDt * P.RT, mad2(av[2], Uf, av[3], Vf), sf);
     }
-    const R uu = Uf * Uf + Vf * Vf;
-    const T a2 = mk2(P.ah_f, P.h_ah), c2 = mk2(P.tauf * (R(1.) - P.ah_f), P.h_ch);
+    const R uu = mad2(Uf, Uf, Vf, Vf);
+    const T a2 = mk2(P.ah_f, P.h_ah), c2 = mk2(mulr(P.tauf, R(1.) - P.ah_f), P.h_ch);
     // face distributions of the six directions crossing the face (three opposite
     // pairs): Eq + a (bh - Eq) + c S
     T out[9];
@@ -567,7 +588,7 @@ __device__ __forceinline__ void face_state_flux(const PR<R> &P, const typename P
     auto face_pair = [&](auto QC) {
         constexpr int Qa = decltype(QC)::value, Qb = Qa + 4;
         T Eq, So, Eqb, Sob;
-        eq_pair<MODEL, Qa>(P, es, Eq, So, Eqb, Sob);
+        eq_pair<MODEL, Qa, XF>(P, es, Eq, So, Eqb, Sob);
         out[Qa] = fma2(c2, So, fma2(a2, sub2(bh[Qa], Eq), Eq));
         out[Qb] = fma2(c2, Sob, fma2(a2, sub2(bh[Qb], Eqb), Eqb));
     };

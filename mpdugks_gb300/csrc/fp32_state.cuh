@@ -28,14 +28,20 @@ struct PR {
     // from ny up are a neighbour's halo (2 rows of device memory) instead of a
     // wall or the periodic wrap; 0 for a whole grid
     int row0, halo_lo, halo_hi;
-    R phi0, p0, aPhi, bPhi, Kp, RT, invRT, hDt, dt, Lambda0;
-    R Beta, Kappa, PhiL, PhiV, RhoL, Gy;
-    R inv_12dx, inv_12dy, inv_6dd, inv_wI_dphi, inv_RTdt;
+    R aPhi, bPhi, Beta, Kappa, RhoL, Gy, inv_wI_dphi;
     R tauf, aBP_f, ah_f;                       // flow relaxation after the first step
     R h_aBP, h_bBP, h_cBP, h_ah, h_bh, h_ch;  // phase-field relaxation
-    R r_2dy, r_ndx, r_n2dx, r_ndy;             // reconstruction multipliers
-    R aTP, bTP, dtV;
     R hneq;  // NEE: 2 TauMass / (2 TauMass + dt), the phase field's non-equilibrium factor
+    // What every D2Q9 case has in common (Ark/Constant/ZeroReference.h, ZeroNamespace.h: R0 = 1,
+    // T0 = 1/3, CFL 1/2, MinL = 1, max |xi| = sqrt(3 RT) = 1, phi 0 .. 1), as constants of the
+    // code: products of them fold, no thread forms them again, and the streaming kernel holds
+    // up to eight registers fewer.  512x2048 Rayleigh-Taylor, 200 steps from a host state: 19.85 ->
+    // 19.08 ms; 3072x3072, 100 steps: 71.7 -> 68.5 ms; UW 512x512, 100 steps: 7.95 -> 7.71 ms.
+    static constexpr R p0 = R(1.0), RT = R(1.0 / 3.0), invRT = R(3.0), Lambda0 = R(1.5), Kp = R(1.0 / 3.0 * 9 / 5.0);
+    static constexpr R dt = R(0.5), hDt = R(0.25), dtV = R(0.5), aTP = R(4.0 / 3.0), bTP = R(1.0 / 3.0);
+    static constexpr R PhiL = R(1.0), PhiV = R(0.0);
+    static constexpr R inv_12dx = R(1.0 / 12.0), inv_12dy = inv_12dx, inv_6dd = R(1.0 / 6.0), inv_RTdt = R(6.0);
+    static constexpr R r_2dy = R(0.5), r_ndx = R(-1.0), r_n2dx = R(-0.5), r_ndy = R(-1.0);  // reconstruction
 };
 using P32 = PR<float>;
 
