@@ -38,6 +38,7 @@
 #include "fp32_state.cuh"
 #include "fp32_math.cuh"
 #include "fp32_stream.cuh"
+#include "pdl.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -346,6 +347,7 @@ __device__ __forceinline__ void tile_step(const PR<R> &P, const SR<R> &S, int fi
 template <int MODEL, bool WALLS, typename R>
 __global__ void __launch_bounds__(BX *BY, 1) k_step32(PR<R> P, SR<R> S, int first, int gin, int gout,
                                                       uint32_t step, int ntx, int ntiles) {
+    pdl_wait();
     constexpr bool PF = prefetched<R>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Views<R> sv(smem_raw);
@@ -751,7 +753,7 @@ static cudaError_t launch_t(const PR<R> &P, const SR<R> &S, int first, int gin, 
     }
     const int ntx = (P.nx + TW - 1) / TW, nty = (P.ny + TH - 1) / TH, ntiles = ntx * nty;
     const dim3 blk(BX, BY);
-    k_step32<MODEL, WALLS, R><<<min(ntiles, nsm), blk, bytes, st>>>(P, S, first, gin, gout, step, ntx, ntiles);
+    launch_pdl(k_step32<MODEL, WALLS, R>, min(ntiles, nsm), blk, bytes, st, P, S, first, gin, gout, step, ntx, ntiles);
     return cudaGetLastError();
 }
 

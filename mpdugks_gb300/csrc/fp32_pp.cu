@@ -29,6 +29,7 @@
 #include <cstdint>
 
 #include "fp32_pp.cuh"
+#include "pdl.cuh"
 
 namespace dugks {
 namespace f32 {
@@ -50,6 +51,7 @@ __device__ __forceinline__ void iso_grad(const PPP &P, const float *__restrict__
 // previous update's psi) when do_msrc, else the stored force; f-bar-plus remainders.
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_pp32_collide(PPP P, PPS S, int do_msrc) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= P.nx || j >= P.ny) return;
     constexpr int Q = PPQ<MODEL>::Q;
@@ -80,6 +82,7 @@ __global__ void __launch_bounds__(256) k_pp32_collide(PPP P, PPS S, int do_msrc)
 // Ark/Cpp/PseudoP.cpp:23-30), stored relative to e_q times the face average of rho.
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_pp32_faces1(PPP P, PPS S) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     const bool xf = blockIdx.z == 0;
     if (i >= P.nx || j >= P.ny) return;
@@ -175,6 +178,7 @@ __device__ __forceinline__ void pp_face2_at(const PPP &P, const PPS &S, int i, i
 // sums, rho in FP64.
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_pp32_faces2u(PPP P, PPS S) {
+    pdl_wait();
     constexpr int Q = PPQ<MODEL>::Q;
     __shared__ float xs[Q][8][33];  // x-face fluxes of the tile's rows, columns 0 .. 32
     __shared__ float ys[Q][9][32];  // y-face fluxes of the tile's columns, rows 0 .. 8
@@ -267,9 +271,15 @@ static cudaError_t launch_pp_t(const PPP &P, const PPS &S, int do_msrc, cudaStre
     const dim3 blk(32, 8);
     const dim3 grd((P.nx + 31) / 32, (P.ny + 7) / 8), grf(grd.x, grd.y, 2);
     (void)step;
-    k_pp32_collide<MODEL><<<grd, blk, 0, st>>>(P, S, do_msrc);
-    k_pp32_faces1<MODEL><<<grf, blk, 0, st>>>(P, S);
-    k_pp32_faces2u<MODEL><<<grd, blk, 0, st>>>(P, S);
+    // programmatic launches, except where a launch has about one block for each of the 152 SMs:
+    // blocks placed before the kernel ahead of them ends then share an SM while others have
+    // none (D2V16, 200 steps: 141x217 cells, 140 blocks, 4.72 ms plain, 4.97 programmatic;
+    // 200x200, 175 blocks, 5.75 / 5.12; 150x150, 95 blocks, 4.53 / 4.36)
+    const unsigned blocks = grd.x * grd.y;
+    const bool early = blocks <= 96 || blocks > 152;
+    launch_after(early, k_pp32_collide<MODEL>, grd, blk, 0, st, P, S, do_msrc);
+    launch_after(early, k_pp32_faces1<MODEL>, grf, blk, 0, st, P, S);
+    launch_after(early, k_pp32_faces2u<MODEL>, grd, blk, 0, st, P, S);
     *launches += 3;
     return cudaGetLastError();
 }

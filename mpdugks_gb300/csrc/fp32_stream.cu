@@ -11,6 +11,7 @@
 
 // constants, ring layouts, TMA helpers shared with the batched streaming kernel
 #include "fp32_stream.cuh"
+#include "pdl.cuh"
 
 namespace dugks {
 namespace f32 {
@@ -30,6 +31,7 @@ template <int MODEL, bool WALLS, bool TMA, bool NEE>
 __global__ void __launch_bounds__(WPB * 32, STREAM_MIN_BLOCKS)
     k_stream32(P32 P, S32 S, int first, int gin, int gout, uint32_t step, int nstrips, int nsegs, int seg_rows,
                const __grid_constant__ CUtensorMap tmap, int zin, int *err) {
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     float *wbase = reinterpret_cast<float *>(smem_raw) + (size_t)wib * WARP_F;
@@ -132,12 +134,12 @@ static cudaError_t launch_stream_t(const P32 &P, const S32 &S, int first, int gi
     const int items = nstrips * nsegs;
     const int blocks = min((items + WPB - 1) / WPB, g_stream_nsm * g_stream_blocks);
     if (tmap) {
-        k_stream32<MODEL, WALLS, true, NEE><<<blocks, WPB * 32, STREAM_SMEM, st>>>(P, S, first, gin, gout, step,
+        launch_pdl(k_stream32<MODEL, WALLS, true, NEE>, blocks, WPB * 32, STREAM_SMEM, st, P, S, first, gin, gout, step,
                                                                                  nstrips, nsegs, seg, *tmap, zin, err);
     } else {
         CUtensorMap none;
         memset(&none, 0, sizeof none);
-        k_stream32<MODEL, WALLS, false, NEE><<<blocks, WPB * 32, STREAM_SMEM, st>>>(P, S, first, gin, gout, step,
+        launch_pdl(k_stream32<MODEL, WALLS, false, NEE>, blocks, WPB * 32, STREAM_SMEM, st, P, S, first, gin, gout, step,
                                                                                   nstrips, nsegs, seg, none, 0, err);
     }
     return cudaGetLastError();

@@ -26,6 +26,7 @@
 #include <cstdint>
 
 #include "fp32_math.cuh"
+#include "pdl.cuh"
 
 namespace dugks {
 namespace f32 {
@@ -74,6 +75,7 @@ __device__ __forceinline__ void load_cell(const S32 &S, size_t c, float2 (&Pq)[9
 // averaged-field inputs (A) and, HCZ, the MacroSource outputs the next step reads.
 template <int MODEL>
 __global__ void __launch_bounds__(UBX *UBY) k_uw32_collide(P32 P, S32 S, float *U, int first) {
+    pdl_wait();
     Cells k;
     if (!cell_of(P, k)) return;
     const size_t qs = S.qs, c = k.c;
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(UBX *UBY) k_uw32_collide(P32 P, S32 S, float *
 // set the pace); the first third also the phase field's.
 constexpr int UW_GRAD_SLICES = 3;
 __global__ void __launch_bounds__(UBX *UBY) k_uw32_grad(P32 P, S32 S, float *U) {
+    pdl_wait();
     Cells k;
     if (!cell_of(P, k)) return;
     const size_t qs = S.qs, c = k.c;
@@ -211,6 +214,7 @@ __device__ __forceinline__ void uw_face(const P32 &P, const S32 &S, float *U, si
 // launch slice per face direction)
 template <int MODEL>
 __global__ void __launch_bounds__(UBX *UBY) k_uw32_faces(P32 P, S32 S, float *U) {
+    pdl_wait();
     Cells k;
     if (!cell_of(P, k)) return;
     uw_face<MODEL, true>(P, S, U, at(P, k.j, k.im), k.c);
@@ -220,6 +224,7 @@ __global__ void __launch_bounds__(UBX *UBY) k_uw32_faces(P32 P, S32 S, float *U)
 // finite-volume update of every cell from its four faces' fluxes
 template <int MODEL>
 __global__ void __launch_bounds__(UBX *UBY) k_uw32_update(P32 P, S32 S, const float *U) {
+    pdl_wait();
     Cells k;
     if (!cell_of(P, k)) return;
     const size_t qs = S.qs, c = k.c;
@@ -255,10 +260,10 @@ __global__ void __launch_bounds__(UBX *UBY) k_uw32_update(P32 P, S32 S, const fl
 template <int MODEL>
 static cudaError_t launch_uw32_t(const P32 &P, const S32 &S, float *U, int first, cudaStream_t st) {
     const dim3 blk(UBX, UBY), grd((P.nx + UBX - 1) / UBX, (P.ny + UBY - 1) / UBY);
-    k_uw32_collide<MODEL><<<grd, blk, 0, st>>>(P, S, U, first);
-    k_uw32_grad<<<dim3(grd.x, grd.y, UW_GRAD_SLICES), blk, 0, st>>>(P, S, U);
-    k_uw32_faces<MODEL><<<grd, blk, 0, st>>>(P, S, U);
-    k_uw32_update<MODEL><<<grd, blk, 0, st>>>(P, S, U);
+    launch_pdl(k_uw32_collide<MODEL>, grd, blk, 0, st, P, S, U, first);
+    launch_pdl(k_uw32_grad, dim3(grd.x, grd.y, UW_GRAD_SLICES), blk, 0, st, P, S, U);
+    launch_pdl(k_uw32_faces<MODEL>, grd, blk, 0, st, P, S, U);
+    launch_pdl(k_uw32_update<MODEL>, grd, blk, 0, st, P, S, U);
     return cudaGetLastError();
 }
 

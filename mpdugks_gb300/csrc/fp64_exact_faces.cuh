@@ -122,6 +122,7 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
 
 template <int MODEL, bool WALLS, bool UW>
 __global__ void __launch_bounds__(256) k_faces_ac(Params P, State S) {
+    pdl_wait();
     int i, j;
     bool xf, lo;
     if (!face_of_thread(P, WALLS, UW, i, j, xf, lo)) return;
@@ -210,6 +211,7 @@ __device__ __forceinline__ void face_pp1(const Params &P, const State &S, int i,
 }
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_faces_pp1(Params P, State S) {
+    pdl_wait();
     int i, j;
     bool xf, lo;
     if (!face_of_thread(P, false, false, i, j, xf, lo)) return;
@@ -255,6 +257,7 @@ __device__ __forceinline__ void face_pp2(const Params &P, const State &S, int i,
 }
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_faces_pp2(Params P, State S) {
+    pdl_wait();
     int i, j;
     bool xf, lo;
     if (!face_of_thread(P, false, false, i, j, xf, lo)) return;
@@ -268,6 +271,7 @@ __global__ void __launch_bounds__(256) k_faces_pp2(Params P, State S) {
 // Ark/Lib/D2Q9HCZ.cpp:133-182, Ark/Lib/D2Q9PP.cpp:89-109).
 template <int MODEL, bool WALLS>
 __global__ void __launch_bounds__(256) k_update(Params P, State S) {
+    pdl_wait();
     int i, j;
     if (!cell_of_thread(P, i, j)) return;
     constexpr int Q = MODEL == PP16 ? 16 : 9;

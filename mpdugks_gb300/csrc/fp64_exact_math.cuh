@@ -287,6 +287,7 @@ __device__ __forceinline__ double src_dot(int xu, int xv, double sx_, double sy_
 // (Ark/Cpp/PseudoP.cpp:31-38) first.
 template <int MODEL, bool WALLS>
 __global__ void __launch_bounds__(256) k_collide(Params P, State S, int do_msrc, int gin, int gout) {
+    pdl_wait();
     int i, j;
     if (!cell_of_thread(P, i, j)) return;
     const int pitch = P.pitch;

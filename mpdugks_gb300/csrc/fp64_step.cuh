@@ -20,6 +20,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "dugks_device.cuh"
+#include "pdl.cuh"
 
 #ifndef DUGKS_EXACT
 #error "define DUGKS_EXACT before including fp64_step.cuh"
@@ -132,6 +133,11 @@ __device__ __forceinline__ bool face_of_thread(const Params &P, bool walls, bool
     i = (int)(t - (unsigned)j * nx);
     return (unsigned)j < (xf ? ny : yrows);
 }
+// Programmatic launches (pdl.cuh) only while every SM quarter has at most one warp of cells:
+// blocks that are placed before the kernel ahead of them ends go to the SMs that finish first,
+// and on larger grids that unevenness costs more FP64 pipe time than the launches saved
+// (333x257 HCZ, FMA: 7.93 ms plain, 9.33 programmatic; 256x256 D2V16 5.54 / 5.85).
+static bool early_launch(const Params &P) { return pad32((unsigned)P.nx * P.ny) <= 32u * 152u * 4u; }
 struct Launch {
     dim3 grid, block;
 };
@@ -175,6 +181,7 @@ __device__ __forceinline__ double cellv(const double *__restrict__ a, int ny, in
 // 6 _2dx, in the reference's operand order.
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_grad6(Params P, State S) {
+    pdl_wait();
     int i, j;
     if (!cell_of_thread(P, i, j)) return;
     const int pitch = P.pitch;
@@ -280,6 +287,7 @@ __device__ __forceinline__ double face_uw(const Params &P, const double *__restr
 // 2 tau / (2 tau + dt); then Wall_3_BB.
 template <int MODEL>
 __global__ void __launch_bounds__(256) k_faces_nee(Params P, State S) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, side = blockIdx.y;
     if (i >= P.nx) return;
     const int ny = P.ny, pitch = P.pitch, jc = side ? ny - 1 : 0;
@@ -334,6 +342,7 @@ __global__ void __launch_bounds__(256) k_faces_nee(Params P, State S) {
 // handing the fields to the host).
 template <int MODEL, bool WALLS>
 __global__ void __launch_bounds__(256) k_finalize(Params P, State S, int gin) {
+    pdl_wait();
     int i, j;
     if (!cell_of_thread(P, i, j)) return;
     const size_t c = (size_t)j * P.pitch + i;
@@ -429,39 +438,41 @@ template <int MODEL, bool WALLS>
 static void launch_step_t(const Params &P, const State &S, int do_msrc, int gin, int gout, cudaStream_t st,
                           int64_t *launches, cudaEvent_t *ev) {
     const auto [grd, blk] = cell_launch(P);
+    const bool early = early_launch(P);
     if (ev) cudaEventRecord(ev[0], st);
-    k_collide<MODEL, WALLS><<<grd, blk, 0, st>>>(P, S, do_msrc, gin, gout);
+    launch_after(early, k_collide<MODEL, WALLS>, grd, blk, 0, st, P, S, do_msrc, gin, gout);
     if (ev) cudaEventRecord(ev[1], st);
     if constexpr (MODEL == AC || MODEL == HCZ) {
         if (!WALLS && P.uw) {  // UW: cell gradients, then the faces with the low-side boundary faces
-            k_grad6<MODEL><<<grd, blk, 0, st>>>(P, S);
+            launch_after(early, k_grad6<MODEL>, grd, blk, 0, st, P, S);
             const auto [gf, bf] = face_launch(P, false, true);
-            k_faces_ac<MODEL, false, true><<<gf, bf, 0, st>>>(P, S);
+            launch_after(early, k_faces_ac<MODEL, false, true>, gf, bf, 0, st, P, S);
             *launches += 4;
         } else {
             const auto [gf, bf] = face_launch(P, WALLS, false);
-            k_faces_ac<MODEL, WALLS, false><<<gf, bf, 0, st>>>(P, S);
+            launch_after(early, k_faces_ac<MODEL, WALLS, false>, gf, bf, 0, st, P, S);
             *launches += 3;
             if (WALLS && P.nee) {  // NEE wall faces over the bounce-back ones
-                k_faces_nee<MODEL><<<dim3((P.nx + 127) / 128, 2), 128, 0, st>>>(P, S);
+                launch_after(early, k_faces_nee<MODEL>, dim3((P.nx + 127) / 128, 2), 128, 0, st, P, S);
                 *launches += 1;
             }
         }
     } else {
         const auto [gf, bf] = face_launch(P, false, false);
-        k_faces_pp1<MODEL><<<gf, bf, 0, st>>>(P, S);
-        k_faces_pp2<MODEL><<<gf, bf, 0, st>>>(P, S);
+        launch_after(early, k_faces_pp1<MODEL>, gf, bf, 0, st, P, S);
+        launch_after(early, k_faces_pp2<MODEL>, gf, bf, 0, st, P, S);
         *launches += 4;
     }
     if (ev) cudaEventRecord(ev[2], st);
-    k_update<MODEL, WALLS><<<grd, blk, 0, st>>>(P, S);
+    launch_after(early, k_update<MODEL, WALLS>, grd, blk, 0, st, P, S);
     if (ev) cudaEventRecord(ev[3], st);
 }
 
 template <int MODEL, bool WALLS>
 static void launch_finalize_t(const Params &P, const State &S, int gin, cudaStream_t st) {
     const auto [grd, blk] = cell_launch(P);
-    k_finalize<MODEL, WALLS><<<grd, blk, 0, st>>>(P, S, gin);
+    const bool early = early_launch(P);
+    launch_after(early, k_finalize<MODEL, WALLS>, grd, blk, 0, st, P, S, gin);
 }
 
 void launch_fp64_step(const Params &P, const State &S, int do_msrc, int gin, int gout, cudaStream_t st,
