@@ -259,9 +259,9 @@ static void split_ff(double v, float &hi, float &lo) {
     lo = (float)(v - (double)hi);
 }
 
-// The D2V16 equilibria (pp_deq, fp32_pp.cuh; d2v16_eq, fp64_step.cuh) skip the inverse
-// moment matrix's structural zeros, and the FP32 and FP64-FMA ones evaluate it by
-// opposite-direction pairs: check that this case's matrix has that form (opposite rows
+// The D2V16 equilibria (pp_deq, fp32_pp.cuh; d2v16_eq, fp64_*_math.cuh) skip the inverse
+// moment matrix's structural zeros, and evaluate it by the parts even and odd in the
+// velocity: check that this case's matrix has that form (opposite rows
 // equal in the even moments' entries, negated in the odd ones; zeros where d2v16_entry
 // says), so a change of the table cannot go unnoticed.
 static bool d2v16_matrix_has_pair_form(const double (&iM)[16][16]) {
@@ -351,16 +351,20 @@ static int create_pp32(dugks_handle *h, dugks_handle_t **out) {
     C.aTP = (float)P.aTP;
     C.bTP = (float)P.bTP;
     C.dtV = (float)P.dtV;
-    C.r_2dy = (float)P.r_2dy;
-    C.r_ndx = (float)P.r_ndx;
-    C.r_n2dx = (float)P.r_n2dx;
-    C.r_ndy = (float)P.r_ndy;
+    C.hc = (float)(P.hDt * P.c16);
+    C.hc2 = 2.f * C.hc;
+    C.hDt2 = 0.5f * C.hDt;
+    {
+        // in FP32, one from the other: where a cell's force and its pressure gradient nearly
+        // balance, the ratio of the source's and the relaxation's rounded factors decides what is left
+        const float tau = C.Tau0, aBP = (2.f * tau - C.hDt) / (2.f * tau + C.dt);
+        C.bBP = 1.f - aBP;
+        C.cBP = tau * C.bBP;
+        C.ah = 2.f * tau / (2.f * tau + C.hDt);
+        C.ch = tau * (1.f - C.ah);
+    }
     C.inv_6_2dx = (float)(1.0 / (P._2dx * 6));
     C.inv_6_2dy = (float)(1.0 / (P._2dy * 6));
-    C.R0 = P.R0;
-    C.T_CS = P.T_CS;
-    C.aCS = P.aCS;
-    C.RTd = P.RT;
     split_ff(P.R0 * P.T_CS, C.rtcs_hi, C.rtcs_lo);
     split_ff(P.aCS, C.acs_hi, C.acs_lo);
     split_ff(P.RT, C.rt_hi, C.rt_lo);
@@ -375,9 +379,19 @@ static int create_pp32(dugks_handle *h, dugks_handle_t **out) {
         pp_rest_eq(P, h->iM, 1.0, rest);
         for (int q = 0; q < Q; ++q) C.erest[q] = (float)rest[q];
     }
-    // this case's inverse moment matrix in FP32 (zeros for D2Q9PP)
-    for (int j = 0; j < 16; ++j)
-        for (int k = 0; k < 16; ++k) C.iM16[j][k] = P.model == PP16 ? (float)h->iM[j][k] : 0.f;
+    if (P.model == PP16) {  // this case's equilibrium coefficients (pp_deq, fp32_pp.cuh)
+        const D2V16Matrix &A = P.m16;
+        const double RT = P.RT;
+        const double k[25] = {A.A + A.G, A.A + A.H, A.T, 7 * RT, A.N * RT,
+                              A.B + A.I + 4.5 * A.S * RT, A.S / 2, A.F - 7 * A.S * RT, -A.S,
+                              A.ic + 3 * A.Pc * RT - 2 * A.N * RT, A.Pc - A.N / 2,
+                              A.D + A.J + RT * (8 * A.U + A.V), A.U, A.D + A.K + RT * (A.U + 8 * A.V), A.V,
+                              RT * (3 * A.Qc + A.R - 0.625 * A.N), A.Qc - A.N / 8, A.R - A.N / 8,
+                              A.E + A.L + 2.25 * A.S * RT, A.S / 4, 1.75 * A.S * RT - A.F / 16, A.S / 4,
+                              RT * (0.3125 * A.N - 0.375 * A.Pc - A.R / 2) - A.jc, A.N / 16 - A.Pc / 8,
+                              A.N / 16 - A.R / 2};
+        for (int j = 0; j < 25; ++j) C.k[j] = (float)k[j];
+    }
     e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         cudaFree(h->arena);

@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) k_pp32_collide(PPP P, PPS S, int do_msrc)
 // moments with the previous face force, face pressure and psi (Ark/Lib/D2Q9PP.cpp:110-136,
 // Ark/Cpp/PseudoP.cpp:23-30), stored relative to e_q times the face average of rho.
 template <int MODEL>
-__global__ void __launch_bounds__(256) k_pp32_faces1(PPP P, PPS S) {
+__global__ void __launch_bounds__(256, MODEL == PP16 ? 4 : 5) k_pp32_faces1(PPP P, PPS S) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     const bool xf = blockIdx.z == 0;
@@ -103,11 +103,9 @@ __global__ void __launch_bounds__(256) k_pp32_faces1(PPP P, PPS S) {
             tn[q] = at(jp, i) - at(jm, i);
             to[q] = at(jp, im) - at(jm, im);
         }
-        const double ravg = 0.5 * (rh(j, im) + rh(j, i));
-        const double hgx = (double)P.hDt * ((rh(j, im) - rh(j, i)) * (double)P.r_ndx);
-        const double hgy =
-            (double)P.hDt * ((0.5 * ((rh(jp, i) - rh(jm, i)) + (rh(jp, im) - rh(jm, im)))) * (double)P.r_2dy);
-        f = pp_face1<MODEL, true>(P, o, n, tn, to, ravg, hgx, hgy, S.xFx[c], S.xFy[c], b);
+        const double ro = rh(j, im), rn = rh(j, i);
+        const float rt = (float)((rh(jp, i) - rh(jm, i)) + (rh(jp, im) - rh(jm, im)));
+        f = pp_face1<MODEL, true>(P, o, n, tn, to, ro + rn, (float)(rn - ro), rt, S.xFx[c], S.xFy[c], b);
     } else {  // between (i, j-1) and (i, j)
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -118,17 +116,16 @@ __global__ void __launch_bounds__(256) k_pp32_faces1(PPP P, PPS S) {
             tn[q] = at(j, im) - at(j, ip);
             to[q] = at(jm, im) - at(jm, ip);
         }
-        const double ravg = 0.5 * (rh(jm, i) + rh(j, i));
-        const double hgx =
-            (double)P.hDt * ((0.5 * ((rh(j, im) - rh(j, ip)) + (rh(jm, im) - rh(jm, ip)))) * (double)P.r_n2dx);
-        const double hgy = (double)P.hDt * ((rh(jm, i) - rh(j, i)) * (double)P.r_ndy);
-        f = pp_face1<MODEL, false>(P, o, n, tn, to, ravg, hgx, hgy, S.yFx[c], S.yFy[c], b);
+        const double ro = rh(jm, i), rn = rh(j, i);
+        const float rt = (float)((rh(j, im) - rh(j, ip)) + (rh(jm, im) - rh(jm, ip)));
+        f = pp_face1<MODEL, false>(P, o, n, tn, to, ro + rn, (float)(rn - ro), rt, S.yFx[c], S.yFy[c], b);
     }
     float *B = xf ? S.xb : S.yb;
 #pragma unroll
     for (int q = 0; q < Q; ++q) B[(size_t)q * S.qs + c] = b[q];
     (xf ? S.xpsl : S.ypsl)[c] = f.psil;
     (xf ? S.xr : S.yr)[c] = f.dr;
+    (xf ? S.xfl : S.yfl)[c] = f.R;
     (xf ? S.xu : S.yu)[c] = f.U;
     (xf ? S.xv : S.yv)[c] = f.V;
     (xf ? S.xg : S.yg)[c] = f.scg;
@@ -155,13 +152,13 @@ __device__ __forceinline__ void pp_face2_at(const PPP &P, const PPS &S, int i, i
     f.dr = (XF ? S.xr : S.yr)[c];
     f.U = (XF ? S.xu : S.yu)[c];
     f.V = (XF ? S.xv : S.yv)[c];
-    const size_t co = XF ? (size_t)j * P.pitch + wrapi(i - 1, P.nx) : (size_t)wrapi(j - 1, P.ny) * P.pitch + i;
-    const float R = (float)(0.5 * (S.rho[co] + S.rho[c]) + (double)f.dr);
+    f.R = (XF ? S.xfl : S.yfl)[c];
     const float *__restrict__ B = XF ? S.xb : S.yb;
     float b[Q];
 #pragma unroll
-    for (int q = 0; q < Q; ++q) b[q] = B[(size_t)q * S.qs + c];
-    pp_face2<MODEL, XF>(P, b, R, f, Fx, Fy, out);
+    for (int q = 0; q < Q; ++q)
+        if ((XF ? lat_u<MODEL>(q) : lat_v<MODEL>(q)) != 0) b[q] = B[(size_t)q * S.qs + c];
+    pp_face2<MODEL, XF>(P, b, f, Fx, Fy, out);
 }
 
 // Face pass 2 and the update (Ark/Cpp/DUGKS2DSolver.cpp:748-792) with the cell macros
@@ -176,8 +173,8 @@ __device__ __forceinline__ void pp_face2_at(const PPP &P, const PPS &S, int i, i
 // px = dt/V (rho_W - rho_E)/2, py = dt/V (rho_S - rho_N)/2 (the e_q avg(rho) flux
 // divergence on unit cells, from the FP64 density); U, V, p, psi from float-float
 // sums, rho in FP64.
-template <int MODEL>
-__global__ void __launch_bounds__(256) k_pp32_faces2u(PPP P, PPS S) {
+template <int MODEL, int MIN_BLOCKS>
+__global__ void __launch_bounds__(256, MIN_BLOCKS) k_pp32_faces2u(PPP P, PPS S) {
     pdl_wait();
     constexpr int Q = PPQ<MODEL>::Q;
     __shared__ float xs[Q][8][33];  // x-face fluxes of the tile's rows, columns 0 .. 32
@@ -191,37 +188,46 @@ __global__ void __launch_bounds__(256) k_pp32_faces2u(PPP P, PPS S) {
     if (in) {
         pp_face2_at<MODEL, true>(P, S, i, j, true, out);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) xs[q][ty][tx] = out[q];
+        for (int q = 0; q < Q; ++q)
+            if (lat_u<MODEL>(q) != 0) xs[q][ty][tx] = out[q];
         pp_face2_at<MODEL, false>(P, S, i, j, true, out);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) ys[q][ty][tx] = out[q];
+        for (int q = 0; q < Q; ++q)
+            if (lat_v<MODEL>(q) != 0) ys[q][ty][tx] = out[q];
     }
     if (t < h) {  // x faces east of the tile (column x0 + w, periodic)
         pp_face2_at<MODEL, true>(P, S, wrapi(x0 + w, P.nx), y0 + t, false, out);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) xs[q][t][w] = out[q];
+        for (int q = 0; q < Q; ++q)
+            if (lat_u<MODEL>(q) != 0) xs[q][t][w] = out[q];
     } else if (t >= 32 && t < 32 + w) {  // y faces north of the tile (row y0 + h, periodic)
         pp_face2_at<MODEL, false>(P, S, x0 + t - 32, wrapi(y0 + h, P.ny), false, out);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) ys[q][h][t - 32] = out[q];
+        for (int q = 0; q < Q; ++q)
+            if (lat_v<MODEL>(q) != 0) ys[q][h][t - 32] = out[q];
     }
     __syncthreads();
     if (!in) return;
     const int pitch = P.pitch;
     const int ip = wrapi(i + 1, P.nx), im = wrapi(i - 1, P.nx), jn = wrapi(j + 1, P.ny), js = wrapi(j - 1, P.ny);
     const size_t c = (size_t)j * pitch + i;
-    const float px = (float)(0.5 * (double)P.dtV * (S.rho[(size_t)j * pitch + im] - S.rho[(size_t)j * pitch + ip]));
-    const float py = (float)(0.5 * (double)P.dtV * (S.rho[(size_t)js * pitch + i] - S.rho[(size_t)jn * pitch + i]));
+    const float hdv = 0.5f * P.dtV;
+    const float px = hdv * (float)(S.rho[(size_t)j * pitch + im] - S.rho[(size_t)j * pitch + ip]);
+    const float py = hdv * (float)(S.rho[(size_t)js * pitch + i] - S.rho[(size_t)jn * pitch + i]);
     float g[Q], bf[Q], fw[Q], fe[Q], fs[Q], fn[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const size_t o = (size_t)q * S.qs;
         g[q] = S.df[o + c];
         bf[q] = S.bf[o + c];
-        fw[q] = xs[q][ty][tx];
-        fe[q] = xs[q][ty][tx + 1];
-        fs[q] = ys[q][ty][tx];
-        fn[q] = ys[q][ty + 1][tx];
+        if (lat_u<MODEL>(q) != 0) {
+            fw[q] = xs[q][ty][tx];
+            fe[q] = xs[q][ty][tx + 1];
+        }
+        if (lat_v<MODEL>(q) != 0) {
+            fs[q] = ys[q][ty][tx];
+            fn[q] = ys[q][ty + 1][tx];
+        }
     }
     const PPCell n = pp_update<MODEL>(P, g, bf, fw, fe, fs, fn, S.rho[c], px, py, S.Fx[c], S.Fy[c]);
 #pragma unroll
@@ -279,7 +285,11 @@ static cudaError_t launch_pp_t(const PPP &P, const PPS &S, int do_msrc, cudaStre
     const bool early = blocks <= 96 || blocks > 152;
     launch_after(early, k_pp32_collide<MODEL>, grd, blk, 0, st, P, S, do_msrc);
     launch_after(early, k_pp32_faces1<MODEL>, grf, blk, 0, st, P, S);
-    launch_after(early, k_pp32_faces2u<MODEL>, grd, blk, 0, st, P, S);
+    // face pass 2 compiled for three (D2Q9: four) resident blocks of 256 threads where the grid
+    // fills them, with more registers for the few blocks of a small one (D2V16, us per step:
+    // 1024x1024 212 / 225, 400x400 35.6 / 38.2, 150x150 17.6 / 15.7; pass 1 for four / five)
+    if (blocks > 2 * 152) launch_after(early, k_pp32_faces2u<MODEL, MODEL == PP16 ? 3 : 4>, grd, blk, 0, st, P, S);
+    else launch_after(early, k_pp32_faces2u<MODEL, 2>, grd, blk, 0, st, P, S);
     *launches += 3;
     return cudaGetLastError();
 }

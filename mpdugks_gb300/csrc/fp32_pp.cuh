@@ -37,57 +37,58 @@ __host__ __device__ constexpr int lat_opp(int q) {
 }
 
 // Equilibrium parts de_q = eq_q(rho, u, v) - e_q rho (zero at rest).
+// D2V16: Macro16 (Ark/Lib/D2V16.cpp:125-145) at T = T0, p = rho RT, minus its value at
+// (rho, 0, 0) (at rest the moments are linear in rho), times the inverse moment matrix
+// (Ark/Lib/D2V16.cpp:34-52).  A ring's four rows are the sums +- of four parts, even or odd in
+// u and in v, and each part is rho or rho u times a polynomial of u^2, v^2 whose coefficients
+// are combinations of the matrix's entries (PPP::k, formed in FP64 on the host): about 75
+// operations and no cancelling moments, where the matrix by opposite pairs took 108 and the
+// moments 35 before it.  Every rounding is written out, so that each kernel including this
+// evaluates it alike.
 template <int MODEL>
 __device__ __forceinline__ void pp_deq(const PPP &P, float rho, float u, float v, float *de) {
     if (MODEL == PP16) {
-        // Macro16 (Ark/Lib/D2V16.cpp:125-145) at T = T0, p = rho RT, minus its value at
-        // (rho, 0, 0) (at rest the moments are linear in rho); times the case's inverse
-        // moment matrix (Ark/Lib/D2V16.cpp:34-52), a kernel parameter
-        const float RT = P.RT, u2 = u * u, v2 = v * v, s2 = u2 + v2;
-        float M[16];
-        M[0] = 0.f;
-        M[1] = rho * u;
-        M[2] = rho * v;
-        M[3] = rho * s2;
-        M[4] = M[1] * v;
-        M[5] = rho * u2;
-        M[6] = rho * v2;
-        M[7] = M[1] * (5.f * RT + s2);
-        M[8] = M[2] * (5.f * RT + s2);
-        M[9] = M[1] * (3.f * RT + u2);
-        M[10] = M[2] * (3.f * RT + v2);
-        M[11] = M[2] * (RT + u2);
-        M[12] = M[1] * (RT + v2);
-        M[13] = (7.f * RT + s2) * M[4];
-        M[14] = rho * RT * (8.f * u2 + v2) + rho * u2 * s2;
-        M[15] = rho * RT * (8.f * v2 + u2) + rho * v2 * s2;
-        // row j' (the opposite direction of j) holds row j's entries of the even moments and
-        // the negated entries of the odd ones, and the axis rings' rows have fixed zeros
-        // (d2v16_odd_moment, d2v16_entry): per opposite pair the even and odd partial sums,
-        // de_j = E + O, de_j' = E - O
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int jo = lat_opp<PP16>(j);
-            if (jo < j) continue;
-            float E = 0.f, O = 0.f;
-#pragma unroll
-            for (int k = 1; k < 16; ++k) {
-                if (!d2v16_entry(j, k)) continue;
-                if (d2v16_odd_moment(k)) O = fmaf(P.iM16[j][k], M[k], O);
-                else E = fmaf(P.iM16[j][k], M[k], E);
-            }
-            de[j] = E + O;
-            de[jo] = E - O;
+        const float *k = P.k;
+        const float a = __fmul_rn(u, u), b = __fmul_rn(v, v), s2 = __fadd_rn(a, b);
+        const float M1 = __fmul_rn(rho, u), M2 = __fmul_rn(rho, v), ruv = __fmul_rn(M1, v), rs2 = __fmul_rn(rho, s2);
+        auto ring = [&](int q, float ee, float xy, float ox, float oy) {  // diagonals (1,1) (-1,1) (-1,-1) (1,-1)
+            const float p = __fadd_rn(ee, xy), m = __fsub_rn(ee, xy), c = __fadd_rn(ox, oy), d = __fsub_rn(ox, oy);
+            de[q] = __fadd_rn(p, c);
+            de[q + 2] = __fsub_rn(p, c);
+            de[q + 1] = __fsub_rn(m, d);
+            de[q + 3] = __fadd_rn(m, d);
+        };
+        auto axis = [&](int q, float e0, float e1, float ox, float oy) {  // (1,0) (0,1) (-1,0) (0,-1)
+            de[q] = __fadd_rn(e0, ox);
+            de[q + 2] = __fsub_rn(e0, ox);
+            de[q + 1] = __fadd_rn(e1, oy);
+            de[q + 3] = __fsub_rn(e1, oy);
+        };
+        {
+            const float w = __fmul_rn(__fmul_rn(k[2], __fsub_rn(a, b)), __fadd_rn(k[3], s2));
+            const float e0 = __fmul_rn(rho, fmaf(k[0], a, fmaf(k[1], b, w)));
+            const float e1 = __fmul_rn(rho, fmaf(k[1], a, fmaf(k[0], b, -w)));
+            axis(0, e0, e1, __fmul_rn(k[4], M1), __fmul_rn(k[4], M2));
         }
+        ring(4, __fmul_rn(rs2, fmaf(k[6], s2, k[5])), __fmul_rn(ruv, fmaf(k[8], s2, k[7])),
+             __fmul_rn(M1, fmaf(k[10], a, k[9])), __fmul_rn(M2, fmaf(k[10], b, k[9])));
+        {
+            const float U = fmaf(k[12], s2, k[11]), V = fmaf(k[14], s2, k[13]);
+            axis(8, __fmul_rn(rho, fmaf(a, U, __fmul_rn(b, V))), __fmul_rn(rho, fmaf(b, U, __fmul_rn(a, V))),
+                 __fmul_rn(M1, fmaf(k[16], a, fmaf(k[17], b, k[15]))), __fmul_rn(M2, fmaf(k[16], b, fmaf(k[17], a, k[15]))));
+        }
+        ring(12, __fmul_rn(rs2, fmaf(k[19], s2, k[18])), __fmul_rn(ruv, fmaf(k[21], s2, k[20])),
+             __fmul_rn(M1, fmaf(k[23], a, fmaf(k[24], b, k[22]))), __fmul_rn(M2, fmaf(k[23], b, fmaf(k[24], a, k[22]))));
     } else {
-        // D2Q9PP (Ark/Lib/D2Q9PP.cpp:51-62): w rho (1 + u1 + u1^2/2 - |u|^2 lambda) - w rho;
-        // every rounding written out, so that each kernel including this evaluates it alike
-        const float uu = fmaf(u, u, __fmul_rn(v, v));
+        // D2Q9PP (Ark/Lib/D2Q9PP.cpp:51-62): w rho (1 + u1 + u1^2/2 - |u|^2 lambda) - w rho
+        const float uuL = __fmul_rn(fmaf(u, u, __fmul_rn(v, v)), P.Lambda0);
+        de[0] = -__fmul_rn(__fmul_rn(P.w9[0], rho), uuL);
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
+        for (int q = 1; q <= 4; ++q) {
             const float u1 = __fmul_rn(__fadd_rn(sxf(d2q9_xu(q), u), sxf(d2q9_xv(q), v)), P.invRT);
-            const float t = fmaf(__fmul_rn(0.5f, u1), u1, u1);
-            de[q] = __fmul_rn(P.w9[q], __fmul_rn(rho, fmaf(-uu, P.Lambda0, t)));
+            const float h = fmaf(__fmul_rn(0.5f, u1), u1, -uuL), wr = __fmul_rn(P.w9[q], rho);
+            de[q] = __fmul_rn(wr, __fadd_rn(h, u1));
+            de[q + 4] = __fmul_rn(wr, __fsub_rn(h, u1));
         }
     }
 }
@@ -129,9 +130,10 @@ __device__ __forceinline__ FF ff_mul(FF a, FF b) {
     return fast_two_sum(p, e);
 }
 __device__ __forceinline__ FF ff_div(FF a, FF b) {
-    const float q1 = __fdiv_rn(a.hi, b.hi);
+    // quotient digits from one reciprocal (within an ulp; the second digit corrects the first's)
+    const float y = rcp(b.hi), q1 = __fmul_rn(a.hi, y);
     const FF r = ff_add(a, ff_neg(ff_mul(b, FF{q1, 0.f})));
-    return fast_two_sum(q1, __fdiv_rn(__fadd_rn(r.hi, r.lo), b.hi));
+    return fast_two_sum(q1, __fmul_rn(__fadd_rn(r.hi, r.lo), y));
 }
 __device__ __forceinline__ FF ff_norm(FF a) { return two_sum(a.hi, a.lo); }
 
@@ -155,8 +157,12 @@ __device__ __forceinline__ void cs_psi(const PPP &P, FF rho, FF p, float &scg, f
     const float G = (float)((g.hi > 0.f) - (g.hi < 0.f));
     scg = G;
     const float xh = 2.f * g.hi * G, xl = 2.f * g.lo * G;  // G = +-1: exact
-    psi = sqrtf(xh);
-    psil = psi > 0.f ? __fdiv_rn(fmaf(-psi, psi, xh) + xl, 2.f * psi) : 0.f;
+    // the root and its residual's correction from one reciprocal root y
+    const float y = rsqrtf(xh), hy = __fmul_rn(0.5f, y), r0 = __fmul_rn(xh, y);
+    const float r1 = fmaf(fmaf(-r0, r0, xh), hy, r0);
+    const bool zero = xh == 0.f;
+    psi = zero ? 0.f : r1;
+    psil = zero ? 0.f : __fmul_rn(__fadd_rn(fmaf(-r1, r1, xh), xl), hy);
 }
 __device__ __forceinline__ double ff_to_double(FF a) { return (double)a.hi + (double)a.lo; }
 
@@ -201,7 +207,7 @@ template <int MODEL>
 __device__ __forceinline__ void pp_src_proj(const PPP &P, float fx, float fy, float U, float V,
                                             float (&pr)[PPQ<MODEL>::Q]) {
     constexpr int Q = PPQ<MODEL>::Q;
-    const float w = fmaf(fx, U, fy * V);
+    const float w = fmaf(fx, U, __fmul_rn(fy, V));
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int qo = lat_opp<MODEL>(q);
@@ -210,9 +216,9 @@ __device__ __forceinline__ void pp_src_proj(const PPP &P, float fx, float fy, fl
             pr[q] = -w;
             continue;
         }
-        const float d = fmaf(fx, P.xi_u[q], fy * P.xi_v[q]);
-        pr[q] = d - w;
-        pr[qo] = -d - w;
+        const float d = fmaf(fx, P.xi_u[q], __fmul_rn(fy, P.xi_v[q]));
+        pr[q] = __fsub_rn(d, w);
+        pr[qo] = -__fadd_rn(d, w);
     }
 }
 
@@ -225,16 +231,13 @@ __device__ __forceinline__ void pp_collide(const PPP &P, const float (&g)[PPQ<MO
     constexpr int Q = PPQ<MODEL>::Q;
     float de[Q];
     pp_deq<MODEL>(P, rho, U, V, de);
-    const float tau = P.Tau0;
-    const float aBP = (2.f * tau - P.hDt) / (2.f * tau + P.dt), bBP = 1.f - aBP, cBP = tau * bBP;
-    const float inv = 1.f / (rho * P.RT);
+    const float ci = __fmul_rn(P.cBP, rcp(__fmul_rn(rho, P.RT)));
     float pr[Q];
     pp_src_proj<MODEL>(P, fx, fy, U, V, pr);
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const float eq = fmaf(P.erest[q], rho, de[q]);
-        const float So = pr[q] * eq * inv;
-        bf[q] = g[q] + (bBP * (de[q] - g[q]) + cBP * So);
+        bf[q] = fmaf(P.bBP, __fsub_rn(de[q], g[q]), fmaf(__fmul_rn(pr[q], eq), ci, g[q]));
     }
 }
 
@@ -242,71 +245,83 @@ __device__ __forceinline__ void pp_collide(const PPP &P, const float (&g)[PPQ<MO
 // between o = below and n = above): the half-step reconstruction relative to e_q times the
 // face average of rho, from the f-bar-plus remainders of the two cells (o, n) and the sums
 // tn, to of their tangential differences ((t+) - (t-) of n and of o: x face rows +-1, y face
-// columns -1 minus +1); ravg, hgx, hgy: the density's face average and hDt times its
-// gradient (FP64); (fxp, fyp): the face force of the previous step.  Out: b, the face
-// velocity, the face density relative to ravg (dr) and the face psi pair and sign.
+// columns -1 minus +1).  rsum (FP64), rd, rt: the sum of the two cells' densities, their
+// difference n - o and the sum of their tangential differences taken like tn, to; (fxp, fyp):
+// the face force of the previous step.  Out: b, the face velocity, the face density (R) and
+// it relative to the average (dr), and the face psi pair and sign.
+// A direction's reconstruction is s/2 - hDt xi.grad with the lattice speed in the constants
+// (PPP::hc = hDt c), the components that are zero left out; the e_q rho part's gradient terms
+// are those of four directions, their negatives and doubles.
 struct PPFace {
-    float U, V, dr, psi, psil, scg;
+    float U, V, R, dr, psi, psil, scg;
 };
 template <int MODEL, bool XF>
 __device__ __forceinline__ PPFace pp_face1(const PPP &P, const float (&o)[PPQ<MODEL>::Q],
                                            const float (&n)[PPQ<MODEL>::Q], const float (&tn)[PPQ<MODEL>::Q],
-                                           const float (&to)[PPQ<MODEL>::Q], double ravg, double hgx, double hgy,
+                                           const float (&to)[PPQ<MODEL>::Q], double rsum, float rd, float rt,
                                            float fxp, float fyp, float (&b)[PPQ<MODEL>::Q]) {
     constexpr int Q = PPQ<MODEL>::Q;
-    const float hgxf = (float)hgx, hgyf = (float)hgy;
+    constexpr float T = XF ? 0.25f : -0.25f;  // tangential: a quarter of the sum, along +y / +x
+    const float rn = __fmul_rn(P.hc, rd), rq = __fmul_rn(P.hc, __fmul_rn(T, rt));
+    const float rp = __fadd_rn(rn, rq), rm = __fsub_rn(rn, rq);
     FF sR{0.f, 0.f}, su{0.f, 0.f}, sv{0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        float gx, gy;
-        if (XF) {
-            gy = (0.5f * (tn[q] + to[q])) * P.r_2dy;
-            gx = (o[q] - n[q]) * P.r_ndx;
-        } else {
-            gx = (0.5f * (tn[q] + to[q])) * P.r_n2dx;
-            gy = (o[q] - n[q]) * P.r_ndy;
+        const int nn = XF ? lat_u<MODEL>(q) : lat_v<MODEL>(q), nt = XF ? lat_v<MODEL>(q) : lat_u<MODEL>(q);
+        const bool two = nn * nn > 1 || nt * nt > 1;
+        const float hc = two ? P.hc2 : P.hc, er = two ? 2.f * P.erest[q] : P.erest[q];
+        float bq = __fmul_rn(0.5f, __fadd_rn(o[q], n[q])), r = 0.f;
+        if (nn != 0 && nt != 0) {
+            const bool same = (nn > 0) == (nt > 0);
+            const float g = fmaf(same ? T : -T, __fadd_rn(tn[q], to[q]), __fsub_rn(n[q], o[q]));
+            bq = fmaf(nn > 0 ? -hc : hc, g, bq);
+            r = same ? rp : rm;
+            bq = fmaf(nn > 0 ? -er : er, r, bq);
+        } else if (nn != 0) {
+            bq = fmaf(nn > 0 ? -hc : hc, __fsub_rn(n[q], o[q]), bq);
+            bq = fmaf(nn > 0 ? -er : er, rn, bq);
+        } else if (nt != 0) {
+            bq = fmaf(nt > 0 ? -T * hc : T * hc, __fadd_rn(tn[q], to[q]), bq);
+            bq = fmaf(nt > 0 ? -er : er, rq, bq);
         }
-        float bq = 0.5f * (o[q] + n[q]) - P.hDt * (gx * P.xi_u[q] + gy * P.xi_v[q]);
-        bq = fmaf(-P.erest[q], hgxf * P.xi_u[q] + hgyf * P.xi_v[q], bq);
         b[q] = bq;
         ff_acc(sR, bq);
     }
     pp_first_moments<MODEL>(P, b, su, sv);
     sR = ff_norm(sR);
-    const float rah = (float)ravg;
-    const FF R = ff_add(FF{rah, (float)(ravg - (double)rah)}, sR);
-    const float Rf = R.hi;
+    // the average rsum / 2 as a pair
+    const float rah2 = (float)rsum;
+    const FF R = ff_add(FF{__fmul_rn(0.5f, rah2), __fmul_rn(0.5f, (float)(rsum - (double)rah2))}, sR);
+    const float inv = rcp(R.hi);
     PPFace f;
-    f.U = __fadd_rn(su.hi, su.lo) / Rf;
-    f.V = __fadd_rn(sv.hi, sv.lo) / Rf;
-    f.U += 0.5f * P.hDt * fxp / Rf;
-    f.V += 0.5f * P.hDt * fyp / Rf;
+    f.U = __fmul_rn(fmaf(P.hDt2, fxp, __fadd_rn(su.hi, su.lo)), inv);
+    f.V = __fmul_rn(fmaf(P.hDt2, fyp, __fadd_rn(sv.hi, sv.lo)), inv);
     const FF p = cs_p(P, R);
     cs_psi(P, R, p, f.scg, f.psi, f.psil);
+    f.R = R.hi;
     f.dr = __fadd_rn(sR.hi, sR.lo);  // face rho - avg(rho)
     return f;
 }
 
 // Face pass 2 of one face: equilibrium, source of the face force (fx, fy) and the flux
-// xi.n of the face values relative to e_q avg(rho); R the face density.
+// xi.n of the face values relative to e_q avg(rho), of the directions that cross the face
+// (the others' are not formed).
 template <int MODEL, bool XF>
-__device__ __forceinline__ void pp_face2(const PPP &P, const float (&b)[PPQ<MODEL>::Q], float R, const PPFace &f,
-                                         float fx, float fy, float (&out)[PPQ<MODEL>::Q]) {
+__device__ __forceinline__ void pp_face2(const PPP &P, const float (&b)[PPQ<MODEL>::Q], const PPFace &f, float fx,
+                                         float fy, float (&out)[PPQ<MODEL>::Q]) {
     constexpr int Q = PPQ<MODEL>::Q;
     float de[Q];
-    pp_deq<MODEL>(P, R, f.U, f.V, de);
-    const float tauh = P.Tau0;
-    const float ah = 2.f * tauh / (2.f * tauh + P.hDt), bh = 1.f - ah, ch = tauh * bh;
-    const float inv = 1.f / (R * P.RT);
+    pp_deq<MODEL>(P, f.R, f.U, f.V, de);
+    const float ci = __fmul_rn(P.ch, rcp(__fmul_rn(f.R, P.RT)));
     float pr[Q];
     pp_src_proj<MODEL>(P, fx, fy, f.U, f.V, pr);
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        const float eq = fmaf(P.erest[q], R, de[q]);
-        const float So = pr[q] * eq * inv;
+        if ((XF ? lat_u<MODEL>(q) : lat_v<MODEL>(q)) == 0) continue;
+        const float eq = fmaf(P.erest[q], f.R, de[q]);
         const float heq = fmaf(P.erest[q], f.dr, de[q]);  // eq - e_q avg(rho)
-        const float t = heq + ah * (b[q] - heq) + ch * So;
-        out[q] = t * (XF ? P.xi_u[q] : P.xi_v[q]);
+        const float t = fmaf(__fmul_rn(pr[q], eq), ci, fmaf(P.ah, __fsub_rn(b[q], heq), heq));
+        out[q] = __fmul_rn(t, XF ? P.xi_u[q] : P.xi_v[q]);
     }
 }
 
@@ -329,13 +344,13 @@ __device__ __forceinline__ PPCell pp_update(const PPP &P, float (&g)[PPQ<MODEL>:
     FF sd{0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        float s = 0.f;
-        s += -fe[q];
-        s += -fn[q];
-        s += fw[q];
-        s += fs[q];
+        const int nu = lat_u<MODEL>(q), nv = lat_v<MODEL>(q);
+        float s = 0.f;  // over the faces the direction crosses
+        if (nu != 0 && nv != 0) s = __fadd_rn(__fadd_rn(-__fadd_rn(fe[q], fn[q]), fw[q]), fs[q]);
+        else if (nu != 0) s = __fsub_rn(fw[q], fe[q]);
+        else if (nv != 0) s = __fsub_rn(fs[q], fn[q]);
         sq[q] = s;
-        ff_acc(sd, s);
+        if (nu != 0 || nv != 0) ff_acc(sd, s);
     }
     const double drho = (double)P.dtV * ((double)sd.hi + (double)sd.lo);
     const float drf = (float)drho;
@@ -344,17 +359,16 @@ __device__ __forceinline__ PPCell pp_update(const PPP &P, float (&g)[PPQ<MODEL>:
     FF su{0.f, 0.f}, sv{0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        float inc = fmaf(P.aTP, bf[q] - g[q], P.dtV * sq[q]);
-        inc = fmaf(P.erest[q], (P.xi_u[q] * px + P.xi_v[q] * py) - drf, inc);
-        g[q] = g[q] + inc;
+        float inc = fmaf(P.aTP, __fsub_rn(bf[q], g[q]), __fmul_rn(P.dtV, sq[q]));
+        inc = fmaf(P.erest[q], fmaf(P.xi_u[q], px, fmaf(P.xi_v[q], py, -drf)), inc);
+        g[q] = __fadd_rn(g[q], inc);
     }
     pp_first_moments<MODEL>(P, g, su, sv);
     const float rh = (float)c.rho;
     const FF R{rh, (float)(c.rho - (double)rh)};
-    c.U = __fadd_rn(su.hi, su.lo) / rh;
-    c.V = __fadd_rn(sv.hi, sv.lo) / rh;
-    c.U += P.hDt * fx / rh;
-    c.V += P.hDt * fy / rh;
+    const float inv = rcp(rh);
+    c.U = __fmul_rn(fmaf(P.hDt, fx, __fadd_rn(su.hi, su.lo)), inv);
+    c.V = __fmul_rn(fmaf(P.hDt, fy, __fadd_rn(sv.hi, sv.lo)), inv);
     const FF p = cs_p(P, R);
     cs_psi(P, R, p, c.scg, c.psi, c.psil);
     c.p = ff_to_double(p);

@@ -185,10 +185,8 @@ __global__ void __launch_bounds__(PWPB * 32, 5)
                         tn[q] = BRQ(j + 1, q, lane) - BRQ(j - 1, q, lane);
                         to[q] = BRQ(j + 1, q, lane - 1) - BRQ(j - 1, q, lane - 1);
                     }
-                    const double ravg = 0.5 * (r1w + r1);
-                    const double hgx = (double)P.hDt * ((r1w - r1) * (double)P.r_ndx);
-                    const double hgy = (double)P.hDt * ((0.5 * ((r2 - r0) + (r2w - r0w))) * (double)P.r_2dy);
-                    xn = pp_face1<MODEL, true>(P, o, n, tn, to, ravg, hgx, hgy, xfp.x, xfp.y, b);
+                    const float rt = (float)((r2 - r0) + (r2w - r0w));
+                    xn = pp_face1<MODEL, true>(P, o, n, tn, to, r1w + r1, (float)(r1 - r1w), rt, xfp.x, xfp.y, b);
                     float *d = xbr + (size_t)(j & 1) * Q * 32 + lane;
 #pragma unroll
                     for (int q = 0; q < Q; ++q) d[q * 32] = b[q];
@@ -206,10 +204,8 @@ __global__ void __launch_bounds__(PWPB * 32, 5)
                         tn[q] = BRQ(j, q, lane - 1) - BRQ(j, q, lane + 1);
                         to[q] = BRQ(j - 1, q, lane - 1) - BRQ(j - 1, q, lane + 1);
                     }
-                    const double ravg = 0.5 * (r1 + r2);
-                    const double hgx = (double)P.hDt * ((0.5 * ((r2w - r2e) + (r1w - r1e))) * (double)P.r_n2dx);
-                    const double hgy = (double)P.hDt * ((r1 - r2) * (double)P.r_ndy);
-                    yfn = pp_face1<MODEL, false>(P, o, n, tn, to, ravg, hgx, hgy, yfp.x, yfp.y, b);
+                    const float rt = (float)((r2w - r2e) + (r1w - r1e));
+                    yfn = pp_face1<MODEL, false>(P, o, n, tn, to, r1 + r2, (float)(r2 - r1), rt, yfp.x, yfp.y, b);
                     float *d = ybr + (size_t)(j & 1) * Q * 32 + lane;
 #pragma unroll
                     for (int q = 0; q < Q; ++q) d[q * 32] = b[q];
@@ -234,12 +230,11 @@ __global__ void __launch_bounds__(PWPB * 32, 5)
                         out.xFx[c] = Fx;
                         out.xFy[c] = Fy;
                     }
-                    const float R = (float)(0.5 * (r0w + r0) + (double)x0.dr);
                     float b[Q];
                     const float *s = xbr + (size_t)(k & 1) * Q * 32 + lane;
 #pragma unroll
                     for (int q = 0; q < Q; ++q) b[q] = s[q * 32];
-                    pp_face2<MODEL, true>(P, b, R, x0, Fx, Fy, FW);
+                    pp_face2<MODEL, true>(P, b, x0, Fx, Fy, FW);
                 }
             }
             float FE[Q];
@@ -264,20 +259,20 @@ __global__ void __launch_bounds__(PWPB * 32, 5)
                         out.yFx[c] = Fx;
                         out.yFy[c] = Fy;
                     }
-                    const float R = (float)(0.5 * (r0 + r1) + (double)yf1.dr);
                     float b[Q];
                     const float *s = ybr + (size_t)((k + 1) & 1) * Q * 32 + lane;
 #pragma unroll
                     for (int q = 0; q < Q; ++q) b[q] = s[q * 32];
-                    pp_face2<MODEL, false>(P, b, R, yf1, Fx, Fy, FN);
+                    pp_face2<MODEL, false>(P, b, yf1, Fx, Fy, FN);
                 }
             }
             // ---- update of row k
             const double r0e = shdnd(r0);
             if (k >= y0 && l_upd) {
                 const size_t c = cell(k);
-                const float px = (float)(0.5 * (double)P.dtV * (r0w - r0e));
-                const float py = (float)(0.5 * (double)P.dtV * (rm - r1));
+                const float hdv = 0.5f * P.dtV;
+                const float px = hdv * (float)(r0w - r0e);
+                const float py = hdv * (float)(rm - r1);
                 float g[Q], bf[Q];
                 const float *sl = stg + (size_t)((k + 8) & 3) * Q * 32 + lane;
 #pragma unroll

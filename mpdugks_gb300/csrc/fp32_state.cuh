@@ -103,17 +103,17 @@ __host__ __device__ __forceinline__ size_t gphi_row(int buf, int side) { return 
 struct PPP {
     int nx, ny, pitch, model, Q;
     float hDt, dt, RT, invRT, Lambda0, Tau0, aTP, bTP, dtV;
-    float r_2dy, r_ndx, r_n2dx, r_ndy, inv_6_2dx, inv_6_2dy;
-    double R0, T_CS, aCS, RTd;
+    float inv_6_2dx, inv_6_2dy;
+    float hc, hc2, hDt2;             // hDt times the lattice speed, twice that; hDt / 2
+    float bBP, cBP, ah, ch;          // relaxation of the collision and of the faces
     // the same constants as float-float pairs (hi + lo) for the device arithmetic:
     // R0 T_CS, aCS, RT
     float rtcs_hi, rtcs_lo, acs_hi, acs_lo, rt_hi, rt_lo;
     float lat_hi, lat_lo;  // the lattice speed (velocities = lat times small integers) as hi + lo
     float xi_u[16], xi_v[16], w9[9], erest[16];
-    // D2V16 inverse moment matrix of this case, by value: the kernels read its entries as
-    // constant-bank operands (no loads), and cases of different lattice speed run side by
-    // side with their own
-    float iM16[16][16];
+    // D2V16: coefficients of the equilibrium's polynomials (pp_deq, fp32_pp.cuh), by value:
+    // constant-bank operands, and cases of different lattice speed run side by side with their own
+    float k[25];
 };
 // One copy of the state the single-pass pseudopotential step reads or writes (two
 // copies, swapped after each step: a strip segment reads rows its neighbours write)
@@ -130,8 +130,8 @@ struct PPV {
 // two swap after each step.
 struct PPS {
     float *df, *bf;                  // g and the collision's remainders B_q - e_q rho [Q][ny][pitch]
-    float *xb, *yb, *xfl, *yfl;      // face reconstructions and fluxes [Q][ny][pitch]
-    float *xr, *yr, *xu, *yu, *xv, *yv, *xg, *yg, *xps, *yps;  // face rho, U, V, G, psi
+    float *xb, *yb, *xfl, *yfl;      // face reconstructions [Q][ny][pitch]; face rho (plane 0 of xfl, yfl)
+    float *xr, *yr, *xu, *yu, *xv, *yv, *xg, *yg, *xps, *yps;  // face rho - avg(rho), U, V, G, psi
     float *xFx, *xFy, *yFx, *yFy;    // face forces (kept for the next step's face velocity)
     double *rho, *rho_o, *p, *U, *V; // cell density (read / written by the update), pressure, velocity
     float *psi, *scg, *Fx, *Fy;
