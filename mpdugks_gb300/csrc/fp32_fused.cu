@@ -49,33 +49,39 @@ namespace f32 {
 
 constexpr int TW = 30, TH = 14;  // interior tile
 constexpr int BX = 32, BY = 16;  // threads = tile + halo ring
+// Small grids (k_step32s): tiles of 30 x 6 cells by two groups of 32 x 8 threads, so that more
+// SMs have a tile and the x- and the y-face of a cell are computed at the same time
+constexpr int TH_S = 6;
 
-
-// phi pairs (halo 2), f-bar-plus pairs, south-face flux pairs, averaged fields
-constexpr size_t SMEM_ELEMS = (size_t)2 * (BY + 2) * (BX + 2) + (18 + 6 + 12) * BY * BX;
+// phi pairs (halo 2), f-bar-plus pairs, south-face flux pairs, averaged fields of a tile of
+// th interior rows
+__host__ __device__ constexpr size_t smem_elems_of(int th) {
+    return (size_t)2 * (th + 4) * (BX + 2) + (18 + 6 + 12) * (th + 2) * BX;
+}
 // Prefetch staging (storage type float only): the next tile's own-cell planes
 // (the PL_N planes of a state copy) and the phi pairs of its phi ring, copied
 // asynchronously (cp.async) while the current tile computes.
-constexpr int RING_MAX = 2 * (TW + 4) + 2 * (TH + 2);  // ring cells of a full tile
-constexpr size_t STG_ELEMS = (size_t)PL_N * BY * BX + 2 * RING_MAX;
+__host__ __device__ constexpr int ring_max(int th) { return 2 * (TW + 4) + 2 * (th + 2); }  // ring cells of a full tile
 template <typename R>
-constexpr bool prefetched() { return sizeof(R) == 4; }
+__host__ __device__ constexpr bool prefetched() { return sizeof(R) == 4; }
 template <typename R>
-constexpr size_t smem_elems() { return SMEM_ELEMS + (prefetched<R>() ? STG_ELEMS : 0); }
+constexpr size_t smem_elems(int th = TH) {
+    return smem_elems_of(th) + (prefetched<R>() ? (size_t)PL_N * (th + 2) * BX + 2 * ring_max(th) : 0);
+}
 
 
 // Geometry of tile t as seen by thread (e, r): the tile's interior origin and
 // size, and this thread's extended cell (interior plus a one-cell ring).
-template <bool WALLS>
+template <bool WALLS, int H = TH>
 struct TileCell {
     int x0, y0, w, hh, gi, gj;
     bool act, ghost, real;
     size_t c;
     __device__ __forceinline__ TileCell(int t, int ntx, int e, int r, int nx, int ny, int pitch) {
         x0 = (t % ntx) * TW;
-        y0 = (t / ntx) * TH;
+        y0 = (t / ntx) * H;
         w = min(TW, nx - x0);
-        hh = min(TH, ny - y0);
+        hh = min(H, ny - y0);
         act = (e <= w + 1) && (r <= hh + 1);
         gi = wrapi(x0 + e - 1, nx);
         gj = y0 + r - 1;
@@ -100,21 +106,23 @@ struct TileCell {
     }
 };
 
-// Issue the asynchronous copies of tile t's inputs into the staging area.
-template <int MODEL, bool WALLS>
+// Issue the asynchronous copies of tile t's inputs into the staging area.  GROUPS thread
+// groups share the planes (grp: this thread's).
+template <int MODEL, bool WALLS, int H = TH, int GROUPS = 1>
 __device__ __forceinline__ void prefetch_tile(const PR<float> &P, const SR<float> &S, int t, int ntx, int e, int r,
-                                              int tid, float *stg, float *stg_ring) {
-    const TileCell<WALLS> g(t, ntx, e, r, P.nx, P.ny, P.pitch);
+                                              int grp, float *stg, float *stg_ring) {
+    const TileCell<WALLS, H> g(t, ntx, e, r, P.nx, P.ny, P.pitch);
+    constexpr int BS = (H + 2) * BX, RM = ring_max(H);
     if (g.real) {
         float *d = stg + r * BX + e;
-        constexpr int BS = BY * BX;
         // f, g, phi; the aux planes only for the flow-solving model (AC: u = 0)
         constexpr int NPL = MODEL == AC ? PL_AUX : PL_N;
 #pragma unroll
-        for (int k = 0; k < NPL; ++k) cp_async(d + k * BS, S.df + (size_t)k * S.qs + g.c);
+        for (int k = 0; k < NPL; ++k)
+            if (GROUPS == 1 || k % GROUPS == grp) cp_async(d + k * BS, S.df + (size_t)k * S.qs + g.c);
     }
     const int nr = g.nring();
-    for (int k = tid; k < nr; k += BX * BY) {
+    for (int k = grp * BS + r * BX + e; k < nr; k += GROUPS * BS) {
         int re, rr;
         g.ring(k, re, rr);
         int rj = g.y0 + rr - 1;
@@ -122,50 +130,53 @@ __device__ __forceinline__ void prefetch_tile(const PR<float> &P, const SR<float
         if (!WALLS) rj = wrapi(rj, P.ny);
         const size_t cc = (size_t)rj * P.pitch + wrapi(g.x0 + re - 1, P.nx);
         cp_async(stg_ring + k, S.phi + cc);
-        cp_async(stg_ring + RING_MAX + k, S.phi + S.qs + cc);
+        cp_async(stg_ring + RM + k, S.phi + S.qs + cc);
     }
     cp_async_commit();
 }
 
 // Shared-memory views of one CTA
-template <typename R>
+template <typename R, int H = TH>
 struct Views {
     using T = typename Pair<R>::T;
-    T (*sB)[BY][BX];       // f-bar-plus pairs
-    T (*sFS)[BY][BX];      // south-face flux pairs (6 slots)
-    R (*sA)[BY][BX];       // srcx srcy rhox rhoy fx fy
+    T (*sB)[H + 2][BX];    // f-bar-plus pairs
+    T (*sFS)[H + 2][BX];   // south-face flux pairs (6 slots)
+    R (*sA)[H + 2][BX];    // srcx srcy rhox rhoy fx fy
     T (*sphi)[BX + 2];     // phi pairs (head, tail), halo 2
-    R *stg;                // [PL_N][BY][BX] staged own-cell inputs (prefetch)
-    R *stg_ring;           // [2][RING_MAX] staged ring phi pairs (prefetch)
+    R *stg;                // [PL_N][H + 2][BX] staged own-cell inputs (prefetch)
+    R *stg_ring;           // [2][ring_max(H)] staged ring phi pairs (prefetch)
     __device__ __forceinline__ explicit Views(unsigned char *raw) {
         R *smem = reinterpret_cast<R *>(raw);
-        sB = reinterpret_cast<T(*)[BY][BX]>(smem);
+        sB = reinterpret_cast<T(*)[H + 2][BX]>(smem);
         sFS = sB + 9;
-        sA = reinterpret_cast<R(*)[BY][BX]>(sFS + 6);
-        sphi = reinterpret_cast<T(*)[BX + 2]>(smem + (18 + 12 + 6) * BY * BX);
-        stg = smem + SMEM_ELEMS;
-        stg_ring = stg + PL_N * BY * BX;
+        sA = reinterpret_cast<R(*)[H + 2][BX]>(sFS + 6);
+        sphi = reinterpret_cast<T(*)[BX + 2]>(smem + (18 + 12 + 6) * (H + 2) * BX);
+        stg = smem + smem_elems_of(H);
+        stg_ring = stg + PL_N * (H + 2) * BX;
     }
 };
 
 // One DUGKS step of one tile (stages 0-3).  The caller has made the tile's
 // inputs visible (staged == true: in the staging area) and synchronised the
-// CTA; `hook` runs right after the last read of the staged inputs.
-template <int MODEL, bool WALLS, typename R, typename Hook>
+// CTA; `hook` runs right after the last read of the staged inputs.  GROUPS = 2: the second
+// group of threads (threadIdx.z = 1) computes the y-faces, the first everything else.
+template <int MODEL, bool WALLS, typename R, int H, int GROUPS, typename Hook>
 __device__ __forceinline__ void tile_step(const PR<R> &P, const SR<R> &S, int first, int gin, int gout,
-                                          uint32_t step, const TileCell<WALLS> &g, const Views<R> &sv,
+                                          uint32_t step, const TileCell<WALLS, H> &g, const Views<R, H> &sv,
                                           bool staged, Hook &&hook) {
+    constexpr int BY = H + 2, RM = ring_max(H);
     using T = typename Pair<R>::T;
     const auto sB = sv.sB;
     const auto sFS = sv.sFS;
     const auto sA = sv.sA;
     const auto sphi = sv.sphi;
     const R *stg = sv.stg, *stg_ring = sv.stg_ring;
-    const int e = threadIdx.x, r = threadIdx.y;
-    const int tid = r * BX + e;
+    const int e = threadIdx.x, r = threadIdx.y, grp = GROUPS == 1 ? 0 : threadIdx.z;
+    const int tid = (grp * BY + r) * BX + e;
+    const bool cells = grp == 0;  // this thread's group does the cells and the x-faces
     const int nx = P.nx, ny = P.ny, pitch = P.pitch;
     const int x0 = g.x0, y0 = g.y0, w = g.w, hh = g.hh, gi = g.gi, gj = g.gj;
-    const bool act = g.act, ghost = g.ghost, real = g.real;
+    const bool act = g.act, ghost = g.ghost && cells, real = g.real && cells;
     const size_t c = g.c;
 
     // ---- stage 0: own deviations (f, g pairs), phi pairs of the halo-2 region
@@ -183,14 +194,14 @@ __device__ __forceinline__ void tile_step(const PR<R> &P, const SR<R> &S, int fi
         sfz = z.x;
         Pq[0].y = -z.y;  // g_0 = -sum_{q>0} g_q
         sphi[r + 1][e + 1] = mk2(plane(PL_PHI), plane(PL_PHI + 1));
-    } else if (act && WALLS) {
+    } else if (WALLS && act && ghost) {
         // ghost phi: the previous step's extrapolation (Ark/Cpp/Boundary.cpp:38-63)
         const size_t gr = gphi_row(gin, gj < 0 ? 0 : 1);
         sphi[r + 1][e + 1] = mk2(S.gphi[gr * pitch + gi], S.gphi[(gr + 1) * pitch + gi]);
     }
     {   // ring of the phi region
         const int nr = g.nring();
-        for (int k = tid; k < nr; k += BX * BY) {
+        for (int k = tid; k < nr; k += GROUPS * BX * BY) {
             int re, rr;
             g.ring(k, re, rr);
             const int ri = wrapi(x0 + re - 1, nx);
@@ -204,7 +215,7 @@ __device__ __forceinline__ void tile_step(const PR<R> &P, const SR<R> &S, int fi
             } else {
                 if (!WALLS) rj = wrapi(rj, ny);
                 const size_t cc = (size_t)rj * pitch + ri;
-                v = staged ? mk2(stg_ring[k], stg_ring[RING_MAX + k]) : mk2(S.phi[cc], S.phi[S.qs + cc]);
+                v = staged ? mk2(stg_ring[k], stg_ring[RM + k]) : mk2(S.phi[cc], S.phi[S.qs + cc]);
             }
             sphi[rr + 1][re + 1] = v;
         }
@@ -269,8 +280,8 @@ __device__ __forceinline__ void tile_step(const PR<R> &P, const SR<R> &S, int fi
     };
     // ---- stage 2: west x-face and south y-face of this thread's cell
     T FW[6], FSo[6];
-    const bool do_x = act && e >= 1 && r >= 1 && r <= hh;           // faces x0-1|x0 .. x0+w-1|x0+w
-    const bool do_y = act && r >= 1 && e >= 1 && e <= w;            // faces below rows 0..hh (hh+1 with the top)
+    const bool do_x = cells && act && e >= 1 && r >= 1 && r <= hh;                          // faces x0-1|x0 .. x0+w-1|x0+w
+    const bool do_y = (GROUPS == 1 || !cells) && act && r >= 1 && e >= 1 && e <= w;  // faces below rows 0..hh (hh+1 with the top)
     if (do_x) {
         R av[6];
 #pragma unroll
@@ -315,7 +326,10 @@ __device__ __forceinline__ void tile_step(const PR<R> &P, const SR<R> &S, int fi
     if (real && e >= 1 && e <= w && r >= 1 && r <= hh) {
         T FN[6], dn[9];
 #pragma unroll
-        for (int s = 0; s < 6; ++s) FN[s] = sFS[s][r + 1][e];
+        for (int s = 0; s < 6; ++s) {
+            FN[s] = sFS[s][r + 1][e];
+            if (GROUPS == 2) FSo[s] = sFS[s][r][e];
+        }
         const R half_dtv = R(0.5) * P.dtV;
         const R px = half_dtv * pdiff(phiB(r, e - 1), phiB(r, e + 1));
         const R py = half_dtv * pdiff(phiB(r - 1, e), phiB(r + 1, e));
@@ -351,21 +365,41 @@ __global__ void __launch_bounds__(BX *BY, 1) k_step32(PR<R> P, SR<R> S, int firs
     constexpr bool PF = prefetched<R>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Views<R> sv(smem_raw);
-    const int e = threadIdx.x, r = threadIdx.y, tid = r * BX + e;
+    const int e = threadIdx.x, r = threadIdx.y;
     if constexpr (PF) {
-        if ((int)blockIdx.x < ntiles)
-            prefetch_tile<MODEL, WALLS>(P, S, blockIdx.x, ntx, e, r, tid, sv.stg, sv.stg_ring);
+        if ((int)blockIdx.x < ntiles) prefetch_tile<MODEL, WALLS>(P, S, blockIdx.x, ntx, e, r, 0, sv.stg, sv.stg_ring);
     }
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const TileCell<WALLS> g(t, ntx, e, r, P.nx, P.ny, P.pitch);
         if constexpr (PF) cp_async_wait_all();
         __syncthreads();  // staged inputs visible; the previous tile is done with shared memory
-        tile_step<MODEL, WALLS, R>(P, S, first, gin, gout, step, g, sv, PF, [&] {
+        tile_step<MODEL, WALLS, R, TH, 1>(P, S, first, gin, gout, step, g, sv, PF, [&] {
             if constexpr (PF) {
                 if (t + (int)gridDim.x < ntiles)
-                    prefetch_tile<MODEL, WALLS>(P, S, t + gridDim.x, ntx, e, r, tid, sv.stg, sv.stg_ring);
+                    prefetch_tile<MODEL, WALLS>(P, S, t + gridDim.x, ntx, e, r, 0, sv.stg, sv.stg_ring);
             }
         });
+    }
+}
+
+// The same over tiles of 30 x 6 cells by two thread groups (FP32 storage): grids whose 30 x 14
+// tiles leave SMs without one.
+template <int MODEL, bool WALLS>
+__global__ void __launch_bounds__(BX *(TH_S + 2) * 2, 1) k_step32s(P32 P, S32 S, int first, int gin, int gout,
+                                                                    uint32_t step, int ntx, int ntiles) {
+    pdl_wait();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Views<float, TH_S> sv(smem_raw);
+    const int e = threadIdx.x, r = threadIdx.y, grp = threadIdx.z;
+    auto issue = [&](int t) {
+        if (t < ntiles) prefetch_tile<MODEL, WALLS, TH_S, 2>(P, S, t, ntx, e, r, grp, sv.stg, sv.stg_ring);
+    };
+    issue(blockIdx.x);
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const TileCell<WALLS, TH_S> g(t, ntx, e, r, P.nx, P.ny, P.pitch);
+        cp_async_wait_all();
+        __syncthreads();  // staged inputs visible; the previous tile is done with shared memory
+        tile_step<MODEL, WALLS, float, TH_S, 2>(P, S, first, gin, gout, step, g, sv, true, [&] { issue(t + gridDim.x); });
     }
 }
 
@@ -392,14 +426,14 @@ __global__ void __launch_bounds__(BX *BY, 1) k_batch32(const int2 *__restrict__ 
                                                        const int *__restrict__ case_stop) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Views<float> sv(smem_raw);
-    const int e = threadIdx.x, r = threadIdx.y, tid = r * BX + e;
+    const int e = threadIdx.x, r = threadIdx.y;
     auto issue = [&](int t) {
         if (t >= ntiles) return;
         const int2 bt = tiles[t];
         const int sn = case_base[bt.x] + kstep;
         if (sn >= case_stop[bt.x]) return;
         const BatchCase &B = c_batch[bt.x];
-        prefetch_tile<MODEL, WALLS>(B.P, B.S[sn & 1], bt.y, B.ntx, e, r, tid, sv.stg, sv.stg_ring);
+        prefetch_tile<MODEL, WALLS>(B.P, B.S[sn & 1], bt.y, B.ntx, e, r, 0, sv.stg, sv.stg_ring);
     };
     issue(blockIdx.x);
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -414,7 +448,7 @@ __global__ void __launch_bounds__(BX *BY, 1) k_batch32(const int2 *__restrict__ 
         cp_async_wait_all();
         __syncthreads();
         const TileCell<WALLS> g(bt.y, B.ntx, e, r, B.P.nx, B.P.ny, B.P.pitch);
-        tile_step<MODEL, WALLS, float>(B.P, B.S[par], sn == 0, par, par ^ 1, (uint32_t)sn, g, sv, true,
+        tile_step<MODEL, WALLS, float, TH, 1>(B.P, B.S[par], sn == 0, par, par ^ 1, (uint32_t)sn, g, sv, true,
                                        [&] { issue(t + gridDim.x); });
     }
 }
@@ -753,6 +787,26 @@ static cudaError_t launch_t(const PR<R> &P, const SR<R> &S, int first, int gin, 
     }
     const int ntx = (P.nx + TW - 1) / TW, nty = (P.ny + TH - 1) / TH, ntiles = ntx * nty;
     const dim3 blk(BX, BY);
+    if constexpr (sizeof(R) == 4) {
+        // One round of 30x6 tiles takes 4.8 us (HCZ, 128x128; 30x14 tiles 7.2), each further one
+        // 3.4 us (5.8): the small tiles where their rounds cost less.  Measured, 30x6 / 30x14:
+        // 64x64 4.7 / 7.2, 128x128 4.8 / 7.3, 160x160 7.9 / 7.4, 256x256 11.5 / 13.0, 300x300
+        // 14.9 / 13.1 us per step.
+        const int small = ntx * ((P.ny + TH_S - 1) / TH_S);
+        if (17 * ((small + nsm - 1) / nsm) < 29 * ((ntiles + nsm - 1) / nsm)) {
+            const size_t sbytes = smem_elems<float>(TH_S) * sizeof(float);
+            static bool sattr = false;
+            if (!sattr) {
+                cudaError_t e = cudaFuncSetAttribute(k_step32s<MODEL, WALLS>,
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sbytes);
+                if (e != cudaSuccess) return e;
+                sattr = true;
+            }
+            launch_pdl(k_step32s<MODEL, WALLS>, min(small, nsm), dim3(BX, TH_S + 2, 2), sbytes, st, P, S, first, gin,
+                       gout, step, ntx, small);
+            return cudaGetLastError();
+        }
+    }
     launch_pdl(k_step32<MODEL, WALLS, R>, min(ntiles, nsm), blk, bytes, st, P, S, first, gin, gout, step, ntx, ntiles);
     return cudaGetLastError();
 }
