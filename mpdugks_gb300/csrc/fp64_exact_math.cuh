@@ -1,4 +1,10 @@
 // Part of fp64_step.cuh, reference-exact variant: equilibria, sources, the collision and the face reconstruction.
+// A product by the FP64 pipe (IM = false) or the integer pipe (fp64_imul.cuh); bad: see there.
+template <bool IM>
+struct Mul {
+    uint32_t bad = 0;
+    __device__ __forceinline__ double operator()(double a, double b) { return IM ? mul_int(a, b, bad) : a * b; }
+};
 // tests of the bits: a floating-point comparison occupies the FP64 pipe like an addition
 __device__ __forceinline__ bool is_zero(double d) { return ((__double2hiint(d) & 0x7fffffff) | __double2loint(d)) == 0; }
 // d = 0 where |d| < 1e-14 (Ark/Header/Mesh_2D.h:196-200)
@@ -265,13 +271,15 @@ __device__ __forceinline__ void hcz_products(MomHCZ &m, double U, double V, doub
     m.cvR[2] = d * Ry;
 }
 // Gamma of both directions; ge: the rest direction's -|u|^2 Lambda0
-__device__ __forceinline__ void hcz_gamma(const MomHCZ &m, double u1, double &G, double &Go) {
-    const double w2 = u1 * u1;
+template <typename M>
+__device__ __forceinline__ void hcz_gamma(M &mul, const MomHCZ &m, double u1, double &G, double &Go) {
+    const double w2 = mul(u1, u1);
     G = __fma_rn(0.5, w2, u1) - m.uuL;
     Go = __fma_rn(0.5, w2, -u1) - m.uuL;
 }
-__device__ __forceinline__ double hcz_source(const MomHCZ &m, double RT, double G, int xu, int xv) {
-    return (1 + G) * (m.cuF[xu + 1] + m.cvF[xv + 1]) + G * RT * (m.cuR[xu + 1] + m.cvR[xv + 1]);
+template <typename M>
+__device__ __forceinline__ double hcz_source(M &mul, const MomHCZ &m, double RT, double G, int xu, int xv) {
+    return mul(1 + G, m.cuF[xu + 1] + m.cvF[xv + 1]) + mul(mul(G, RT), m.cuR[xu + 1] + m.cvR[xv + 1]);
 }
 // (xi.src) of one direction: sum and difference of the components shared by the diagonals
 __device__ __forceinline__ double src_dot(int xu, int xv, double sx_, double sy_, double sum, double dif) {
@@ -285,8 +293,8 @@ __device__ __forceinline__ double src_dot(int xu, int xv, double sx_, double sy_
 // Ark/Cpp/DUGKS2DSolver.cpp:379-401); PP: Ark/Lib/D2Q9PP.cpp:51-62,137-145.
 // do_msrc: run the previous step's MacroSource / pseudopotential cell force
 // (Ark/Cpp/PseudoP.cpp:31-38) first.
-template <int MODEL, bool WALLS>
-__global__ void __launch_bounds__(256) k_collide(Params P, State S, int do_msrc, int gin, int gout) {
+template <int MODEL, bool WALLS, bool IM>
+__global__ void __launch_bounds__(256, IM ? 2 : 1) k_collide(Params P, State S, int do_msrc, int gin, int gout) {
     pdl_wait();
     int i, j;
     if (!cell_of_thread(P, i, j)) return;
@@ -335,7 +343,7 @@ __global__ void __launch_bounds__(256) k_collide(Params P, State S, int do_msrc,
         const double ssum = srcx + srcy, sdif = srcy - srcx;
         // f-bar-plus and h-bar-plus of direction q from its equilibria and sources; hc: the
         // product h_cBP hSo (opposite directions: the negative)
-        auto put = [&](int q, double fEq, double fSo, double hEq, double hSo, double hc) {
+        auto put = [&](auto &mul, int q, double fEq, double fSo, double hEq, double hSo, double hc) {
             const size_t o = (size_t)q * S.qs + c;
             if (WALLS && P.nee && (j == 0 || j == P.ny - 1)) {  // kept for the NEE wall faces
                 const size_t wq = ((size_t)(j == 0 ? 0 : 1) * 9 + q) * pitch + i, ws = (size_t)2 * 9 * pitch;
@@ -344,42 +352,49 @@ __global__ void __launch_bounds__(256) k_collide(Params P, State S, int do_msrc,
                 S.weq[2 * ws + wq] = hEq;
                 S.weq[3 * ws + wq] = hSo;
             }
-            const double hb = P.h_aBP * S.h[o] + P.h_bBP * hEq;
+            const double hb = mul(P.h_aBP, S.h[o]) + mul(P.h_bBP, hEq);
             S.bh[o] = q == 0 ? hb : hb + hc;
-            S.bf[o] = aBP * S.f[o] + bBP * fEq + cBP * fSo;
+            S.bf[o] = mul(aBP, S.f[o]) + mul(bBP, fEq) + mul(cBP, fSo);
         };
+        Mul<false> fp;
         {   // rest direction: u1 = 0, no phase source
             const double w = d2q9_w(0);
             if (MODEL == AC) {  // u = v = 0 (Ark/Lib/D2Q9AC.cpp:197-198): Gamma = 0, no force term
                 const size_t o = c;
                 const double fEq = w * pRT - pRT, hEq = w * phi;
-                if (WALLS && P.nee && (j == 0 || j == P.ny - 1)) put(0, fEq, 0.0, hEq, 0.0, 0.0);
+                if (WALLS && P.nee && (j == 0 || j == P.ny - 1)) put(fp, 0, fEq, 0.0, hEq, 0.0, 0.0);
                 else {
                     S.bh[o] = P.h_aBP * S.h[o] + P.h_bBP * hEq;
                     S.bf[o] = aBP * S.f[o] + bBP * fEq;
                 }
             } else {
                 const double G = -m.uuL;
-                put(0, w * (p + rho * G * P.RT), w * hcz_source(m, P.RT, G, 0, 0), w * phi, 0.0, 0.0);
+                put(fp, 0, w * (p + rho * G * P.RT), w * hcz_source(fp, m, P.RT, G, 0, 0), w * phi, 0.0, 0.0);
             }
         }
 #pragma unroll
         for (int q = 1; q <= 4; ++q) {
             const int xu = d2q9_xu(q), xv = d2q9_xv(q), qo = d2q9_bb(q);
             const double w = d2q9_w(q);
-            const double hSo = src_dot(xu, xv, srcx, srcy, ssum, sdif) * w, hc = P.h_cBP * hSo;
-            if (MODEL == AC) {
-                const double hEq = w * phi, fEq = w * pRT, fSo = w * fr.get(xu, xv);
-                put(q, fEq, fSo, hEq, hSo, hc);
-                put(qo, fEq, -fSo, hEq, -hSo, -hc);
-            } else {
-                const double u1 = m.ur.get(xu, xv);
-                double G, Go;
-                hcz_gamma(m, u1, G, Go);
-                put(q, w * (p + rho * G * P.RT), w * hcz_source(m, P.RT, G, xu, xv), w * (1.0 + u1) * phi, hSo, hc);
-                put(qo, w * (p + rho * Go * P.RT), w * hcz_source(m, P.RT, Go, -xu, -xv), w * (1.0 - u1) * phi, -hSo,
-                    -hc);
-            }
+            auto pair = [&](auto &mul) {
+                const double hSo = mul(src_dot(xu, xv, srcx, srcy, ssum, sdif), w), hc = mul(P.h_cBP, hSo);
+                if (MODEL == AC) {
+                    const double hEq = mul(w, phi), fEq = mul(w, pRT), fSo = mul(w, fr.get(xu, xv));
+                    put(mul, q, fEq, fSo, hEq, hSo, hc);
+                    put(mul, qo, fEq, -fSo, hEq, -hSo, -hc);
+                } else {
+                    const double u1 = m.ur.get(xu, xv);
+                    double G, Go;
+                    hcz_gamma(mul, m, u1, G, Go);
+                    put(mul, q, mul(w, p + mul(mul(rho, G), P.RT)), mul(w, hcz_source(mul, m, P.RT, G, xu, xv)),
+                        mul(mul(w, 1.0 + u1), phi), hSo, hc);
+                    put(mul, qo, mul(w, p + mul(mul(rho, Go), P.RT)), mul(w, hcz_source(mul, m, P.RT, Go, -xu, -xv)),
+                        mul(mul(w, 1.0 - u1), phi), -hSo, -hc);
+                }
+            };
+            Mul<IM> mul;
+            pair(mul);
+            if (IM && mul.bad) pair(fp);  // an operand beyond the integer product's window
         }
     } else {
         double fx, fy;

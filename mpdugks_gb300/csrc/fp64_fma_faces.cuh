@@ -138,7 +138,7 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
     }
 }
 
-template <int MODEL, bool WALLS, bool UW>
+template <int MODEL, bool WALLS, bool UW, bool IM>
 __global__ void __launch_bounds__(256) k_faces_ac(Params P, State S) {
     pdl_wait();
     int i, j;

@@ -181,7 +181,7 @@ __device__ __forceinline__ void macro_source(const Params &P, const State &S, in
 // Ark/Cpp/DUGKS2DSolver.cpp:379-401); PP: Ark/Lib/D2Q9PP.cpp:51-62,137-145.
 // do_msrc: run the previous step's MacroSource / pseudopotential cell force
 // (Ark/Cpp/PseudoP.cpp:31-38) first.
-template <int MODEL, bool WALLS>
+template <int MODEL, bool WALLS, bool IM>
 __global__ void __launch_bounds__(256) k_collide(Params P, State S, int do_msrc, int gin, int gout) {
     pdl_wait();
     int i, j;

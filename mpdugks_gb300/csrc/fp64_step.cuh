@@ -20,6 +20,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "dugks_device.cuh"
+#include "fp64_imul.cuh"
 #include "pdl.cuh"
 
 #ifndef DUGKS_EXACT
@@ -138,6 +139,14 @@ __device__ __forceinline__ bool face_of_thread(const Params &P, bool walls, bool
 // and on larger grids that unevenness costs more FP64 pipe time than the launches saved
 // (333x257 HCZ, FMA: 7.93 ms plain, 9.33 programmatic; 256x256 D2V16 5.54 / 5.85).
 static bool early_launch(const Params &P) { return pad32((unsigned)P.nx * P.ny) <= 32u * 152u * 4u; }
+// Products of the collision and the faces by the integer pipe (fp64_imul.cuh): the exact
+// variant on grids large enough for 32 x 8 blocks.  A face's 359 FP64 instructions become 277,
+// the collision's 373 become 250, and both kernels stay at 70-81 % of the pipe's issue rate.
+// The code is four times as long, and the one-warp blocks of a smaller grid do not run through
+// it together.  us per step, without / with: 256x256 174 / 170, 400x400 412 / 430, 1000x1000
+// 2437 / 2059.  (Taken out again: the quotients' and moments' products too, which spilled, and
+// the update's, 154 registers: 2289.)
+static bool integer_products(const Params &P) { return pad32((unsigned)P.nx) * P.ny >= BAND_THREADS; }
 struct Launch {
     dim3 grid, block;
 };
@@ -440,17 +449,21 @@ static void launch_step_t(const Params &P, const State &S, int do_msrc, int gin,
     const auto [grd, blk] = cell_launch(P);
     const bool early = early_launch(P);
     if (ev) cudaEventRecord(ev[0], st);
-    launch_after(early, k_collide<MODEL, WALLS>, grd, blk, 0, st, P, S, do_msrc, gin, gout);
+    constexpr bool CAN_IM = DUGKS_EXACT && (MODEL == AC || MODEL == HCZ);
+    const bool im = CAN_IM && integer_products(P);
+    if (im) launch_after(early, k_collide<MODEL, WALLS, CAN_IM>, grd, blk, 0, st, P, S, do_msrc, gin, gout);
+    else launch_after(early, k_collide<MODEL, WALLS, false>, grd, blk, 0, st, P, S, do_msrc, gin, gout);
     if (ev) cudaEventRecord(ev[1], st);
     if constexpr (MODEL == AC || MODEL == HCZ) {
         if (!WALLS && P.uw) {  // UW: cell gradients, then the faces with the low-side boundary faces
             launch_after(early, k_grad6<MODEL>, grd, blk, 0, st, P, S);
             const auto [gf, bf] = face_launch(P, false, true);
-            launch_after(early, k_faces_ac<MODEL, false, true>, gf, bf, 0, st, P, S);
+            launch_after(early, k_faces_ac<MODEL, false, true, false>, gf, bf, 0, st, P, S);
             *launches += 4;
         } else {
             const auto [gf, bf] = face_launch(P, WALLS, false);
-            launch_after(early, k_faces_ac<MODEL, WALLS, false>, gf, bf, 0, st, P, S);
+            if (im) launch_after(early, k_faces_ac<MODEL, WALLS, false, CAN_IM>, gf, bf, 0, st, P, S);
+            else launch_after(early, k_faces_ac<MODEL, WALLS, false, false>, gf, bf, 0, st, P, S);
             *launches += 3;
             if (WALLS && P.nee) {  // NEE wall faces over the bounce-back ones
                 launch_after(early, k_faces_nee<MODEL>, dim3((P.nx + 127) / 128, 2), 128, 0, st, P, S);

@@ -23,3 +23,14 @@ def run_check(tmp_path, source: str, n: int):
 
 def test_shared_reciprocal_quotient_is_the_ieee_quotient(tmp_path):
     run_check(tmp_path, 'qdiv_check.c', 20_000_000)
+
+
+def test_integer_product_is_the_ieee_product(tmp_path):
+    gxx = shutil.which('g++')
+    if gxx is None:
+        pytest.skip('g++ not available')
+    exe = tmp_path / 'imul_check'
+    subprocess.run([gxx, '-O2', '-std=c++17', '-ffp-contract=off', '-o', str(exe), str(HERE / 'imul_check.cpp')],
+                   check=True)
+    r = subprocess.run([str(exe), '20000000'], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip().endswith(' 0 mismatches'), r.stdout
