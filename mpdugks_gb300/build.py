@@ -22,8 +22,8 @@ NVFLAGS = ['-O3', '-lineinfo', '-std=c++17', '-Xcompiler', '-fPIC', '-Xcompiler'
            '-Xcompiler', '-ffp-contract=off', '--expt-relaxed-constexpr', f'-I{INCLUDE}']
 
 
-# the reference-exact FP64 step keeps every multiply and add separately rounded
-PER_FILE = {'fp64_exact.cu': ['-fmad=false']}
+# the reference-exact FP64 step and the initial states keep every multiply and add separately rounded
+PER_FILE = {'fp64_exact.cu': ['-fmad=false'], 'init.cu': ['-fmad=false']}
 
 
 def sources() -> list[Path]:

@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -84,6 +85,15 @@ using exact::launch_reduce;
 using exact::launch_check_finite;
 void build_d2v16_matrix(double c, double out[16][16]);
 void derive_params(const dugks_case_t &cs, const dugks_grid_t &g, Params &P);
+int host_init_plane(const Params &P, int kind, const double *params, int nparams, uint64_t seed, double *out);
+double init_rest_f(const Params &P, int q);
+cudaError_t launch_init64(const Params &P, const State &S, const double *f9, const double iM[16][16], cudaStream_t st,
+                          int64_t *launches);
+template <typename R>
+cudaError_t launch_init_dev(const Params &P, const f32::SR<R> &S, const double *field, const double *df9, cudaStream_t st,
+                            int64_t *launches);
+cudaError_t launch_init_pp32(const Params &P, const f32::PPP &C, const f32::PPS &S, const double iM[16][16],
+                             cudaStream_t st, int64_t *launches);
 int host_init_state(const Params &P, const double iM[16][16], int kind, const double *params, int nparams,
                     uint64_t seed, std::vector<double> &f, std::vector<double> &h, std::vector<double> &aux);
 void pp_rest_eq(const Params &P, const double iM[16][16], double rho, double *eq);
@@ -840,13 +850,67 @@ extern "C" int dugks_gpu_upload(dugks_handle_t *h, const double *f, const double
     return DUGKS_OK;
 }
 
+// The state an upload of host_init_state's planes would leave, made on the device from the
+// initialisation's field (init.cu).
+static int init_state(dugks_handle *h, int kind, const double *params, int nparams, uint64_t seed) {
+    const Params &P = h->P;
+    const size_t n = (size_t)P.nx * P.ny;
+    const bool hasH = (P.model == AC || P.model == HCZ);
+    std::unique_ptr<double[]> field(new (std::nothrow) double[n]);
+    if (!field) return fail(h, DUGKS_ENOMEM, "host allocation failed");
+    int rc = host_init_plane(P, kind, params, nparams, seed, field.get());
+    if (rc) return fail(h, rc, "unknown init kind or bad parameters for this model");
+    if ((rc = sync_last(h))) return rc;
+    cudaStream_t st = h->last_stream;
+    const size_t cellb = align256((size_t)P.pitch * sizeof(double) * P.ny);
+    cudaError_t e = cudaSuccess;
+    auto clear = [&](void *p, size_t bytes) {
+        if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, bytes, st);
+    };
+    // the field's plane: the phase field or density itself, or (deviation storage) an output plane
+    double *plane = h->S.fld[h->fp32 || !hasH ? F_RHO : F_PHI];
+    if (!h->fp32 && !h->pp32)
+        for (int k = 0; k < NFIELDS; ++k) clear(h->S.fld[k], cellb);
+    if (e == cudaSuccess)
+        e = cudaMemcpy2DAsync(plane, (size_t)P.pitch * sizeof(double), field.get(), (size_t)P.nx * sizeof(double),
+                              (size_t)P.nx * sizeof(double), P.ny, cudaMemcpyHostToDevice, st);
+    clear(h->rho_last, (size_t)P.pitch * P.ny * sizeof(double));
+    double f9[9], df9[9];
+    for (int q = 0; q < 9 && hasH; ++q) {
+        f9[q] = init_rest_f(P, q);
+        df9[q] = f9[q] - f_rest(P, q);
+    }
+    if (h->pp32) {
+        f32::PPS &S = h->PPs;
+        float *zero[] = {S.Fx, S.Fy, S.xFx, S.xFy, S.yFx, S.yFy, S.psi, S.scg, S.psil, S.xpsl, S.ypsl};
+        for (auto z : zero) clear(z, S.qs * sizeof(float));
+        if (e == cudaSuccess) e = launch_init_pp32(P, h->PPc, S, h->iM, st, &h->launches);
+    } else if (h->fused64) {
+        if (e == cudaSuccess) e = launch_init_dev<double>(P, h->S64f, plane, df9, st, &h->launches);
+    } else if (h->fp32) {
+        if (e == cudaSuccess) e = launch_init_dev<float>(P, h->S32, plane, df9, st, &h->launches);
+    } else {
+        if (!hasH) {
+            double *pf[] = {h->S.xfFx, h->S.xfFy, h->S.yfFx, h->S.yfFy};
+            for (auto p : pf) clear(p, cellb);
+        }
+        if (e == cudaSuccess) e = launch_init64(P, h->S, f9, h->iM, st, &h->launches);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail(h, e, "initialisation");
+    h->first = 1;
+    h->gcur = 0;
+    h->steps = 0;
+    h->pending = 0;
+    h->pp_pending = 0;
+    h->macros_fresh = false;
+    return DUGKS_OK;
+}
+
 extern "C" int dugks_gpu_init(dugks_handle_t *h, int kind, const double *params, int nparams, uint64_t seed) {
     dugks::TraceRange trace("dugks_gpu_init");
     if (!h) return fail(nullptr, DUGKS_EINVAL, "null handle");
-    std::vector<double> f, hd, aux;
-    int rc = host_init_state(h->P, h->iM, kind, params, nparams, seed, f, hd, aux);
-    if (rc) return fail(h, rc, "unknown init kind or bad parameters for this model");
-    rc = dugks_gpu_upload(h, f.data(), hd.empty() ? nullptr : hd.data(), aux.data());
+    int rc = init_state(h, kind, params, nparams, seed);
     if (rc == DUGKS_OK) {
         h->init_kind = kind;
         h->init_radius = (nparams >= 1 && params && params[0] >= 0) ? params[0] : 0.36 * h->P.nx;

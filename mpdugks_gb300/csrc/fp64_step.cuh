@@ -83,7 +83,7 @@ __host__ __device__ constexpr int vel_u(int q) { return MODEL == PP16 ? d2v16_xu
 template <int MODEL>
 __host__ __device__ constexpr int vel_v(int q) { return MODEL == PP16 ? d2v16_xv(q) : d2q9_xv(q); }
 
-// Cells and faces of a launch.  Grids below BAND_THREADS threads: one-warp blocks whose threads
+// Cells and faces of a launch.  Small grids (wide_blocks): one-warp blocks whose threads
 // run over the cells in row order without regard to the rows' ends, so only the last warp has
 // idle lanes (a warp occupies the FP64 pipe alike however many lanes are active) and the
 // warps spread evenly over the SMs (a lone warp issues an FP64 instruction every 64 cycles,
@@ -95,7 +95,6 @@ __host__ __device__ constexpr int vel_v(int q) { return MODEL == PP16 ? d2v16_xv
 // Passes of the benchmark's sizes, 32x8 blocks / one-warp blocks: 32x24 AC 2.67 / 1.86 ms, 128x128
 // AC 2.72 / 2.29, 256x256 D2V16 6.16 / 5.49, 333x257 HCZ (FMA) 9.49 / 8.16, 512x2048 HCZ 15.94 /
 // 16.27.
-constexpr unsigned BAND_THREADS = 32u * 152u * 100u;
 __device__ __forceinline__ bool cell_of_thread(const Params &P, int &i, int &j) {
     if (blockDim.y > 1) {
         i = blockIdx.x * 32 + threadIdx.x;
@@ -139,6 +138,15 @@ __device__ __forceinline__ bool face_of_thread(const Params &P, bool walls, bool
 // and on larger grids that unevenness costs more FP64 pipe time than the launches saved
 // (333x257 HCZ, FMA: 7.93 ms plain, 9.33 programmatic; 256x256 D2V16 5.54 / 5.85).
 static bool early_launch(const Params &P) { return pad32((unsigned)P.nx * P.ny) <= 32u * 152u * 4u; }
+// 32 x 8 blocks: from 486 k cells, or from 230 k where the integer products run with them (us
+// per step, one-warp blocks without / 32 x 8 with: 400x400 412 / 429, 460x460 519 / 521, 500x500
+// 609 / 589, 600x600 875 / 802)
+static bool im_model(const Params &P) { return DUGKS_EXACT && (P.model == AC || P.model == HCZ) && !P.uw; }
+static bool wide_blocks(const Params &P) {
+    const unsigned nx = P.nx;
+    if (16 * pad32(nx) > 17 * nx) return false;  // columns that leave many lanes of a row idle
+    return pad32(nx) * P.ny >= (im_model(P) ? 230400u : 32u * 152u * 100u);
+}
 // Products of the collision and the faces by the integer pipe (fp64_imul.cuh): the exact
 // variant on grids large enough for 32 x 8 blocks.  A face's 359 FP64 instructions become 277,
 // the collision's 373 become 250, and both kernels stay at 70-81 % of the pipe's issue rate.
@@ -146,18 +154,18 @@ static bool early_launch(const Params &P) { return pad32((unsigned)P.nx * P.ny) 
 // it together.  us per step, without / with: 256x256 174 / 170, 400x400 412 / 430, 1000x1000
 // 2437 / 2059.  (Taken out again: the quotients' and moments' products too, which spilled, and
 // the update's, 154 registers: 2289.)
-static bool integer_products(const Params &P) { return pad32((unsigned)P.nx) * P.ny >= BAND_THREADS; }
+static bool integer_products(const Params &P) { return im_model(P) && wide_blocks(P); }
 struct Launch {
     dim3 grid, block;
 };
 static Launch cell_launch(const Params &P) {
     const unsigned nx = P.nx, ny = P.ny;
-    if (pad32(nx) * ny >= BAND_THREADS) return {dim3((nx + 31) / 32, (ny + 7) / 8), dim3(32, 8)};
+    if (wide_blocks(P)) return {dim3((nx + 31) / 32, (ny + 7) / 8), dim3(32, 8)};
     return {dim3(pad32(nx * ny) / 32), dim3(32)};
 }
 static Launch face_launch(const Params &P, bool walls, bool uw) {
     const unsigned nx = P.nx, ny = P.ny, yrows = walls ? ny + 1 : ny;
-    if (pad32(nx) * ny >= BAND_THREADS) return {dim3((nx + 31) / 32, (yrows + 7) / 8, uw ? 4 : 2), dim3(32, 8)};
+    if (wide_blocks(P)) return {dim3((nx + 31) / 32, (yrows + 7) / 8, uw ? 4 : 2), dim3(32, 8)};
     return {dim3((pad32(nx * ny) + pad32(nx * yrows) + (uw ? pad32(ny) + pad32(nx) : 0)) / 32), dim3(32)};
 }
 

@@ -6,8 +6,10 @@
 // device sees the same doubles the reference binary computes.
 // host_init_state runs the reference initialisation functions' steps
 // (Ark/Cpp/Preprocess.cpp) on the SoA layout.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <thread>
 #include <vector>
 
 #include "../../include/dugks_gpu.h"
@@ -222,81 +224,46 @@ void pp_rest_eq(const Params &P, const double iM[16][16], double rho, double *eq
     }
 }
 
-// kind: 0 AC_Drop, 1 droplet heavy inside, 2 Rayleigh-Taylor, 3 SCMP_Drop, 4 density noise.
-int host_init_state(const Params &P, const double iM[16][16], int kind, const double *params, int nparams,
-                    uint64_t seed, std::vector<double> &f, std::vector<double> &h, std::vector<double> &aux) {
-    const int nx = P.nx, ny = P.ny, Q = P.Q;
-    const size_t n = (size_t)nx * ny;
+// x -> a x + c mod 2^64 (Knuth MMIX), k steps at once
+static uint64_t lcg_after(uint64_t x, uint64_t k) {
+    uint64_t a = 6364136223846793005ULL, c = 1442695040888963407ULL, A = 1, C = 0;
+    for (; k; k >>= 1) {
+        if (k & 1) {
+            A = a * A;
+            C = a * C + c;
+        }
+        c = a * c + c;
+        a = a * a;
+    }
+    return A * x + C;
+}
+static double lcg_next(uint64_t &x) {  // uniform in [-1, 1)
+    x = x * 6364136223846793005ULL + 1442695040888963407ULL;
+    const double u01 = (double)(x >> 11) * (1.0 / 9007199254740992.0);
+    return 2.0 * u01 - 1.0;
+}
+
+// The field an initialisation sets, [ny][nx]: the phase field (kinds 0 AC_Drop, 1 droplet heavy
+// inside, 2 Rayleigh-Taylor) or the density (3 SCMP_Drop, 4 density noise); everything else
+// follows from it and the fluid at rest.  Rows in parallel: a row's values do not depend on
+// how the rows are divided (the generator is advanced to each row's first cell).
+int host_init_plane(const Params &P, int kind, const double *params, int nparams, uint64_t seed, double *out) {
+    const int nx = P.nx, ny = P.ny;
     const bool ac = (P.model == AC || P.model == HCZ);
     if (ac && (kind < 0 || kind > 2)) return DUGKS_EINVAL;
     if (!ac && (kind < 3 || kind > 4)) return DUGKS_EINVAL;
-    f.assign((size_t)Q * n, 0.0);
-    h.clear();
-    aux.assign((size_t)NFIELDS * n, 0.0);
-    auto A = [&](int fld, int j, int i) -> double & { return aux[(size_t)fld * n + (size_t)j * nx + i]; };
     const double ChLength = (double)nx, Lx = (double)nx;
-    // MacroQuantity init(Rho0,U0,V0,p0,T0,Lambda0,Mu0): everything else zero
-    const double Rho0 = 1.0, U0 = 0.0, V0 = U0, p0 = 1, Mu0 = P.Tau0 * P.RT * Rho0;  // Mu0 = Nu0*Rho0
-    (void)Mu0;
-    if (ac) {
-        h.assign((size_t)Q * n, 0.0);
-        const double centerX = 0.5 * ChLength, centerY = 0.5 * ChLength;
-        const double radius = (nparams >= 1 && params && params[0] >= 0) ? params[0] : 0.36 * ChLength;
-        // Rayleigh-Taylor interface y = Lx (yc + amp cos(2 pi x / Lx)); optional params
-        // {yc, amp, noise}: mean height and amplitude in units of Lx (default 2, 0.1), and
-        // the amplitude of seeded uniform white noise added to phi (default 0)
-        double rt_yc = 2.0, rt_amp = 0.1, rt_noise = 0.0;
-        if (kind == 2 && params) {
-            if (nparams >= 1) rt_yc = params[0];
-            if (nparams >= 2) rt_amp = params[1];
-            if (nparams >= 3) rt_noise = params[2];
-        }
-        uint64_t rng = seed;
-        // Mu0 of the reference header, not Tau0*RT: the first step's tau is Mu0/(Rho*RT)
-        const double mu0 = P.NuL * Rho0;  // NuL = Nu0 = Mu0/Rho0
-        for (int j = 0; j < ny; ++j)
-            for (int i = 0; i < nx; ++i) {
-                const double x = i + 0.5, y = j + 0.5;
-                double Phi;
-                if (kind == 0) {  // AnalyticalPhiAC_Drop (Ark/Cpp/Preprocess.cpp:402-438)
-                    Phi = 0.5 * (P.PhiL + P.PhiV) + 0.5 * (P.PhiL - P.PhiV) *
-                          std::tanh((std::sqrt((x - centerX) * (x - centerX) + (y - centerY) * (y - centerY)) - radius) *
-                                    2 / P.wI);
-                } else if (kind == 1) {
-                    const double r = std::sqrt((x - centerX) * (x - centerX) + (y - centerY) * (y - centerY));
-                    Phi = 0.5 * (P.PhiL + P.PhiV) + 0.5 * (P.PhiL - P.PhiV) * std::tanh((radius - r) * 2 / P.wI);
-                } else {
-                    const double yi = Lx * (rt_yc + rt_amp * std::cos(2.0 * 3.141592653589793 * x / Lx));
-                    Phi = 0.5 * (P.PhiL + P.PhiV) + 0.5 * (P.PhiL - P.PhiV) * std::tanh((y - yi) * 2 / P.wI);
-                    if (rt_noise != 0.0) {
-                        rng = rng * 6364136223846793005ULL + 1442695040888963407ULL;  // 64-bit LCG (Knuth MMIX)
-                        const double u01 = (double)(rng >> 11) * (1.0 / 9007199254740992.0);
-                        Phi += rt_noise * (2.0 * u01 - 1.0);
-                    }
-                }
-                const double Rho = P.aPhi * (Phi) + P.bPhi;
-                A(F_PHI, j, i) = Phi;
-                A(F_RHO, j, i) = Rho;
-                A(F_U, j, i) = U0;
-                A(F_V, j, i) = V0;
-                A(F_P, j, i) = p0;
-                A(F_TAU, j, i) = mu0 / (Rho * P.RT);  // calcTau with Mu = Mu0
-                // Update_phi_Eq at u = 0, zero forces; Tilde = Eq
-                const double U = U0, V = V0, uu = U * U + V * V;
-                for (int q = 0; q < Q; ++q) {
-                    const double u1 = (P.xi_u[q] * U + P.xi_v[q] * V) / P.RT;
-                    const double GAMMA = u1 + 0.5 * u1 * u1 - uu * P.Lambda0;
-                    const size_t o = (size_t)q * n + (size_t)j * nx + i;
-                    h[o] = P.omega[q] * (1.0 + u1) * (Phi);
-                    if (P.model == AC)
-                        f[o] = P.omega[q] * (p0 / P.RT + Rho * GAMMA) - (double)(!q) * p0 / P.RT;
-                    else
-                        f[o] = P.omega[q] * (p0 + Rho * GAMMA * P.RT);
-                }
-            }
-        return DUGKS_OK;
+    const double centerX = 0.5 * ChLength, centerY = 0.5 * ChLength;
+    const double radius = (nparams >= 1 && params && params[0] >= 0) ? params[0] : 0.36 * ChLength;
+    // Rayleigh-Taylor interface y = Lx (yc + amp cos(2 pi x / Lx)); optional params
+    // {yc, amp, noise}: mean height and amplitude in units of Lx (default 2, 0.1), and
+    // the amplitude of seeded uniform white noise added to phi (default 0)
+    double rt_yc = 2.0, rt_amp = 0.1, rt_noise = 0.0;
+    if (kind == 2 && params) {
+        if (nparams >= 1) rt_yc = params[0];
+        if (nparams >= 2) rt_amp = params[1];
+        if (nparams >= 3) rt_noise = params[2];
     }
-    // pseudopotential
     double rl = 2.4806E-1, rv = 4.5435E-2, prad = 0.25 * ChLength, rho0 = 0.2, amp = 0.01;
     if (kind == 3 && params) {
         if (nparams >= 1) rl = params[0];
@@ -307,37 +274,96 @@ int host_init_state(const Params &P, const double iM[16][16], int kind, const do
         if (nparams >= 1) rho0 = params[0];
         if (nparams >= 2) amp = params[1];
     }
-    uint64_t st = seed;
-    for (int j = 0; j < ny; ++j)
-        for (int i = 0; i < nx; ++i) {
-            const double x = i + 0.5, y = j + 0.5;
-            double Rho;
-            if (kind == 3) {
-                Rho = 0.5 * (rl + rv) - 0.5 * (-rl + rv) *
-                      std::tanh(2 * (std::sqrt((x - 0.5 * ChLength) * (x - 0.5 * ChLength) +
-                                               (y - 0.5 * ChLength) * (y - 0.5 * ChLength)) - prad) / 5.0);
-            } else {
-                st = st * 6364136223846793005ULL + 1442695040888963407ULL;  // 64-bit LCG (Knuth MMIX)
-                const double u01 = (double)(st >> 11) * (1.0 / 9007199254740992.0);
-                Rho = rho0 * (1.0 + amp * (2.0 * u01 - 1.0));
-            }
-            A(F_RHO, j, i) = Rho;
-            A(F_P, j, i) = Rho * P.RT;
-            A(F_U, j, i) = U0;
-            A(F_V, j, i) = V0;
-            A(F_TAU, j, i) = P.Tau0;
-            double eq[16];
-            if (P.model == PP16) {
-                d2v16_eq_host(P, iM, Rho, U0, V0, eq);
-            } else {
-                const double U = U0, V = V0, uu = U * U + V * V;
-                for (int q = 0; q < Q; ++q) {
-                    const double u1 = (P.xi_u[q] * U + P.xi_v[q] * V) / P.RT;
-                    eq[q] = P.omega[q] * Rho * (1.0 + u1 + 0.5 * u1 * u1 - uu * P.Lambda0);
+    const bool noise = (kind == 2 && rt_noise != 0.0) || kind == 4;
+    auto rows = [&](int j0, int j1) {
+        uint64_t rng = noise ? lcg_after(seed, (uint64_t)j0 * (uint64_t)nx) : 0;
+        for (int j = j0; j < j1; ++j)
+            for (int i = 0; i < nx; ++i) {
+                const double x = i + 0.5, y = j + 0.5;
+                double v;
+                if (kind == 0) {  // AnalyticalPhiAC_Drop (Ark/Cpp/Preprocess.cpp:402-438)
+                    v = 0.5 * (P.PhiL + P.PhiV) + 0.5 * (P.PhiL - P.PhiV) *
+                        std::tanh((std::sqrt((x - centerX) * (x - centerX) + (y - centerY) * (y - centerY)) - radius) *
+                                  2 / P.wI);
+                } else if (kind == 1) {
+                    const double r = std::sqrt((x - centerX) * (x - centerX) + (y - centerY) * (y - centerY));
+                    v = 0.5 * (P.PhiL + P.PhiV) + 0.5 * (P.PhiL - P.PhiV) * std::tanh((radius - r) * 2 / P.wI);
+                } else if (kind == 2) {
+                    const double yi = Lx * (rt_yc + rt_amp * std::cos(2.0 * 3.141592653589793 * x / Lx));
+                    v = 0.5 * (P.PhiL + P.PhiV) + 0.5 * (P.PhiL - P.PhiV) * std::tanh((y - yi) * 2 / P.wI);
+                    if (rt_noise != 0.0) v += rt_noise * lcg_next(rng);
+                } else if (kind == 3) {
+                    v = 0.5 * (rl + rv) - 0.5 * (-rl + rv) *
+                        std::tanh(2 * (std::sqrt((x - 0.5 * ChLength) * (x - 0.5 * ChLength) +
+                                                 (y - 0.5 * ChLength) * (y - 0.5 * ChLength)) - prad) / 5.0);
+                } else {
+                    v = rho0 * (1.0 + amp * lcg_next(rng));
                 }
+                out[(size_t)j * nx + i] = v;
             }
-            for (int q = 0; q < Q; ++q) f[(size_t)q * n + (size_t)j * nx + i] = eq[q];
+    };
+    // a thread for every 16 k cells, eight at most
+    const size_t want = std::min<size_t>({8, ((size_t)nx * ny + 16383) / 16384, (size_t)ny,
+                                          std::max<size_t>(1, std::thread::hardware_concurrency())});
+    std::vector<std::thread> pool;
+    int done = 0;
+    try {
+        pool.reserve(want);
+        for (size_t t = 0; t + 1 < want; ++t) {
+            const int next = (int)((t + 1) * (size_t)ny / want);
+            pool.emplace_back(rows, done, next);
+            done = next;
         }
+    } catch (...) {  // no more threads: the rest here
+    }
+    rows(done, ny);
+    for (auto &t : pool) t.join();
+    return DUGKS_OK;
+}
+
+// rest value of f_q in an Allen-Cahn initial state (p = p0 = 1, u = 0)
+double init_rest_f(const Params &P, int q) {
+    const double p0 = 1.0;
+    return P.model == AC ? P.omega[q] * (p0 / P.RT) - (double)(!q) * p0 / P.RT : P.omega[q] * p0;
+}
+
+// The whole state [Q][ny][nx], [ny][nx] planes on the host (slab partitions)
+int host_init_state(const Params &P, const double iM[16][16], int kind, const double *params, int nparams,
+                    uint64_t seed, std::vector<double> &f, std::vector<double> &h, std::vector<double> &aux) {
+    const int Q = P.Q;
+    const size_t n = (size_t)P.nx * P.ny;
+    const bool ac = (P.model == AC || P.model == HCZ);
+    std::vector<double> field(n);
+    const int rc = host_init_plane(P, kind, params, nparams, seed, field.data());
+    if (rc) return rc;
+    f.assign((size_t)Q * n, 0.0);
+    h.clear();
+    // MacroQuantity init(Rho0,U0,V0,p0,T0,Lambda0,Mu0): everything else zero
+    aux.assign((size_t)NFIELDS * n, 0.0);
+    if (ac) h.assign((size_t)Q * n, 0.0);
+    for (size_t c = 0; c < n; ++c) {
+        if (ac) {
+            const double Phi = field[c], Rho = P.aPhi * (Phi) + P.bPhi;
+            aux[F_PHI * n + c] = Phi;
+            aux[F_RHO * n + c] = Rho;
+            aux[F_P * n + c] = 1.0;
+            // Mu0 of the reference header (NuL = Nu0 = Mu0 / Rho0): the first step's tau is Mu0/(Rho*RT)
+            aux[F_TAU * n + c] = P.NuL / (Rho * P.RT);
+            // Update_phi_Eq at u = 0, zero forces; Tilde = Eq
+            for (int q = 0; q < Q; ++q) {
+                h[(size_t)q * n + c] = P.omega[q] * (Phi);
+                f[(size_t)q * n + c] = init_rest_f(P, q);
+            }
+        } else {
+            const double Rho = field[c];
+            aux[F_RHO * n + c] = Rho;
+            aux[F_P * n + c] = Rho * P.RT;
+            aux[F_TAU * n + c] = P.Tau0;
+            double eq[16];
+            pp_rest_eq(P, iM, Rho, eq);
+            for (int q = 0; q < Q; ++q) f[(size_t)q * n + c] = eq[q];
+        }
+    }
     return DUGKS_OK;
 }
 
