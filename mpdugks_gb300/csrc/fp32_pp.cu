@@ -4,9 +4,9 @@
 // the same step (Ark/Cpp/PseudoP.cpp:39-46, Jacobi semantics: all face psi
 // first, then the face forces), so face pass 1 (reconstruction, face moments, face
 // psi) of every face precedes face pass 2 (face force, equilibrium, He-Shan-Doolen
-// source, flux) of any.  Three launches: the collision (with the cell force from the
-// psi of the previous update), face pass 1, and face pass 2 fused with the update (the
-// fluxes of a tile in shared memory; with the cell macros, pressure and psi).
+// source, flux) of any.  Two launches: the collision (with the cell force from the psi of
+// the previous update) with face pass 1, and face pass 2 with the update (the fluxes of a
+// tile in shared memory; with the cell macros, pressure and psi).
 //
 // Storage: the density rho in FP64 and f as the FP32 remainders g_q = f_q - e_q rho,
 // e_q = eq_q(1, 0, 0) the rest equilibrium per unit density.  At rest f = e rho, so
@@ -21,9 +21,7 @@
 // (Fusing face pass 2 with the update saved the fluxes' round trip through DRAM, ~0.2 KB
 // per cell-update, for 0.8 % of the D2V16 step: the passes are latency- as much as
 // bandwidth-bound.  An earlier fusion that recomputed the face reconstruction instead of
-// reading it ran slower, and so did fusing the collision with face pass 1 (f-bar-plus of
-// a 34x10-cell tile ring in shared memory: 127 registers, two blocks per SM, the ring's
-// collisions computed twice; 3.09 against 3.54 G cell-updates/s on D2V16 1024^2).)
+// reading it ran slower.)
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -47,89 +45,123 @@ __device__ __forceinline__ void iso_grad(const PPP &P, const float *__restrict__
     pp_iso_grad(P, at(j, ip), at(j, im), at(jp, i), at(jm, i), at(jp, ip), at(jp, im), at(jm, ip), at(jm, im), gx, gy);
 }
 
-// Collision pre-step: cell force F = -G psi grad psi (Ark/Cpp/PseudoP.cpp:31-38, from the
-// previous update's psi) when do_msrc, else the stored force; f-bar-plus remainders.
-template <int MODEL>
-__global__ void __launch_bounds__(256) k_pp32_collide(PPP P, PPS S, int do_msrc) {
+// Collision and face pass 1 of a 32x8-cell tile by one or two groups of 256 threads.
+// Collision: the cell force F = -G psi grad psi (Ark/Cpp/PseudoP.cpp:31-38, from the previous
+// update's psi) when do_msrc, else the stored force; f-bar-plus remainders to shared memory and
+// to S.bf for the update.  The first group does the tile's cells, the second (or the first
+// again) the ring of one cell around it, which the neighbouring tiles do too, with the same
+// results.
+// Face pass 1, after a block barrier: half-step reconstruction, face moments with the previous
+// face force, face pressure and psi (Ark/Lib/D2Q9PP.cpp:110-136, Ark/Cpp/PseudoP.cpp:23-30),
+// stored relative to e_q times the face average of rho; the first group the west faces of the
+// tile's cells, the second (or the first then) the south faces.
+// As two launches the face pass read the remainders of a face's cells and of their four
+// neighbours from L2 and DRAM, the x and the y faces in different blocks.  Bounded by latency at
+// 16 to 40 warps an SM and, on small grids, by the launches: 150x150 D2V16 15.6 -> 11.8 us a
+// step, D2Q9 15.3 -> 12.0; 1024x1024 214 -> 200 and 148 -> 141.
+template <int MODEL, int GROUPS, int MIN_BLOCKS>
+__global__ void __launch_bounds__(256 * GROUPS, MIN_BLOCKS) k_pp32_faces1(PPP P, PPS S, int do_msrc) {
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= P.nx || j >= P.ny) return;
     constexpr int Q = PPQ<MODEL>::Q;
-    const size_t c = (size_t)j * P.pitch + i;
-    float fx, fy;
-    if (do_msrc) {
-        float gx, gy;
-        iso_grad(P, S.psi, S.psil, i, j, gx, gy);
-        const float k = -S.scg[c] * S.psi[c];
-        fx = gx * k;
-        fy = gy * k;
-        S.Fx[c] = fx;
-        S.Fy[c] = fy;
-    } else {
-        fx = S.Fx[c];
-        fy = S.Fy[c];
-    }
-    float g[Q], bf[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) g[q] = S.df[(size_t)q * S.qs + c];
-    pp_collide<MODEL>(P, g, (float)S.rho[c], (float)S.U[c], (float)S.V[c], fx, fy, bf);
-#pragma unroll
-    for (int q = 0; q < Q; ++q) S.bf[(size_t)q * S.qs + c] = bf[q];
-}
-
-// Face pass 1 (x faces: blockIdx.z = 0, y faces: 1): half-step reconstruction, face
-// moments with the previous face force, face pressure and psi (Ark/Lib/D2Q9PP.cpp:110-136,
-// Ark/Cpp/PseudoP.cpp:23-30), stored relative to e_q times the face average of rho.
-template <int MODEL>
-__global__ void __launch_bounds__(256, MODEL == PP16 ? 4 : 5) k_pp32_faces1(PPP P, PPS S) {
-    pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const bool xf = blockIdx.z == 0;
-    if (i >= P.nx || j >= P.ny) return;
-    constexpr int Q = PPQ<MODEL>::Q;
+    __shared__ float s[Q][10][34];  // f-bar-plus of the tile and its ring
+    const int tx = threadIdx.x, r = threadIdx.y & 7, t = r * 32 + tx;
+    const bool first = threadIdx.y < 8;
+    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 8;
     const int nx = P.nx, ny = P.ny, pitch = P.pitch;
+    const int w = min(32, nx - x0), h = min(8, ny - y0);
+    const bool in = tx < w && r < h;
+    // collides the cell at (cx, cy) from the tile's corner
+    auto collide = [&](int cx, int cy, bool own) {
+        const int i = wrapi(x0 + cx, nx), j = wrapi(y0 + cy, ny);
+        const size_t c = (size_t)j * pitch + i;
+        float g[Q], bf[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) g[q] = S.df[(size_t)q * S.qs + c];
+        float fx, fy;
+        if (do_msrc) {
+            float gx, gy;
+            iso_grad(P, S.psi, S.psil, i, j, gx, gy);
+            const float k = -S.scg[c] * S.psi[c];
+            fx = gx * k;
+            fy = gy * k;
+            if (own) {
+                S.Fx[c] = fx;
+                S.Fy[c] = fy;
+            }
+        } else {
+            fx = S.Fx[c];
+            fy = S.Fy[c];
+        }
+        pp_collide<MODEL>(P, g, (float)S.rho[c], (float)S.U[c], (float)S.V[c], fx, fy, bf);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) s[q][cy + 1][cx + 1] = bf[q];
+        if (own) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) S.bf[(size_t)q * S.qs + c] = bf[q];
+        }
+    };
+    // the ring: its row below (34 cells), its row above (34), its west and its east column (8 each)
+    const int rx = t < 34 ? t - 1 : t < 68 ? t - 35 : t < 76 ? -1 : w;
+    const int ry = t < 34 ? -1 : t < 68 ? h : t < 76 ? t - 68 : t - 76;
+    const bool ring = t < 84 && rx <= w && (t < 68 || ry < h);
+    if (GROUPS == 2) {
+        if (first ? in : ring) collide(first ? tx : rx, first ? r : ry, first);
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k)
+            if (k == 0 ? in : ring) collide(k == 0 ? tx : rx, k == 0 ? r : ry, k == 0);
+    }
+    __syncthreads();
+    if (!in) return;
+    const int i = x0 + tx, j = y0 + r;
     const int im = wrapi(i - 1, nx), ip = wrapi(i + 1, nx), jm = wrapi(j - 1, ny), jp = wrapi(j + 1, ny);
     const size_t c = (size_t)j * pitch + i;
     auto rh = [&](int jj, int ii) { return S.rho[(size_t)jj * pitch + ii]; };
     float o[Q], n[Q], tn[Q], to[Q], b[Q];
-    PPFace f;
-    if (xf) {  // between (i-1, j) and (i, j)
+    if (GROUPS == 1 || first) {  // between (i-1, j) and (i, j)
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            const float *F = S.bf + (size_t)q * S.qs;
-            auto at = [&](int jj, int ii) { return F[(size_t)jj * pitch + ii]; };
-            o[q] = at(j, im);
-            n[q] = at(j, i);
-            tn[q] = at(jp, i) - at(jm, i);
-            to[q] = at(jp, im) - at(jm, im);
+            o[q] = s[q][r + 1][tx];
+            n[q] = s[q][r + 1][tx + 1];
+            tn[q] = s[q][r + 2][tx + 1] - s[q][r][tx + 1];
+            to[q] = s[q][r + 2][tx] - s[q][r][tx];
         }
         const double ro = rh(j, im), rn = rh(j, i);
         const float rt = (float)((rh(jp, i) - rh(jm, i)) + (rh(jp, im) - rh(jm, im)));
-        f = pp_face1<MODEL, true>(P, o, n, tn, to, ro + rn, (float)(rn - ro), rt, S.xFx[c], S.xFy[c], b);
-    } else {  // between (i, j-1) and (i, j)
+        const PPFace f = pp_face1<MODEL, true>(P, o, n, tn, to, ro + rn, (float)(rn - ro), rt, S.xFx[c], S.xFy[c], b);
+#pragma unroll
+        for (int q = 0; q < Q; ++q)  // what face pass 2 reads
+            if (lat_u<MODEL>(q) != 0) S.xb[(size_t)q * S.qs + c] = b[q];
+        S.xpsl[c] = f.psil;
+        S.xr[c] = f.dr;
+        S.xfl[c] = f.R;
+        S.xu[c] = f.U;
+        S.xv[c] = f.V;
+        S.xg[c] = f.scg;
+        S.xps[c] = f.psi;
+    }
+    if (GROUPS == 1 || !first) {  // between (i, j-1) and (i, j)
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            const float *F = S.bf + (size_t)q * S.qs;
-            auto at = [&](int jj, int ii) { return F[(size_t)jj * pitch + ii]; };
-            o[q] = at(jm, i);
-            n[q] = at(j, i);
-            tn[q] = at(j, im) - at(j, ip);
-            to[q] = at(jm, im) - at(jm, ip);
+            o[q] = s[q][r][tx + 1];
+            n[q] = s[q][r + 1][tx + 1];
+            tn[q] = s[q][r + 1][tx] - s[q][r + 1][tx + 2];
+            to[q] = s[q][r][tx] - s[q][r][tx + 2];
         }
         const double ro = rh(jm, i), rn = rh(j, i);
         const float rt = (float)((rh(j, im) - rh(j, ip)) + (rh(jm, im) - rh(jm, ip)));
-        f = pp_face1<MODEL, false>(P, o, n, tn, to, ro + rn, (float)(rn - ro), rt, S.yFx[c], S.yFy[c], b);
-    }
-    float *B = xf ? S.xb : S.yb;
+        const PPFace f = pp_face1<MODEL, false>(P, o, n, tn, to, ro + rn, (float)(rn - ro), rt, S.yFx[c], S.yFy[c], b);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) B[(size_t)q * S.qs + c] = b[q];
-    (xf ? S.xpsl : S.ypsl)[c] = f.psil;
-    (xf ? S.xr : S.yr)[c] = f.dr;
-    (xf ? S.xfl : S.yfl)[c] = f.R;
-    (xf ? S.xu : S.yu)[c] = f.U;
-    (xf ? S.xv : S.yv)[c] = f.V;
-    (xf ? S.xg : S.yg)[c] = f.scg;
-    (xf ? S.xps : S.yps)[c] = f.psi;
+        for (int q = 0; q < Q; ++q)
+            if (lat_v<MODEL>(q) != 0) S.yb[(size_t)q * S.qs + c] = b[q];
+        S.ypsl[c] = f.psil;
+        S.yr[c] = f.dr;
+        S.yfl[c] = f.R;
+        S.yu[c] = f.U;
+        S.yv[c] = f.V;
+        S.yg[c] = f.scg;
+        S.yps[c] = f.psi;
+    }
 }
 
 // Face pass 2 of the x face (XF) or y face at (i, j): face force from the face-psi
@@ -275,22 +307,23 @@ template <int MODEL>
 static cudaError_t launch_pp_t(const PPP &P, const PPS &S, int do_msrc, cudaStream_t st, int64_t *launches,
                                uint32_t step) {
     const dim3 blk(32, 8);
-    const dim3 grd((P.nx + 31) / 32, (P.ny + 7) / 8), grf(grd.x, grd.y, 2);
+    const dim3 grd((P.nx + 31) / 32, (P.ny + 7) / 8);
     (void)step;
-    // programmatic launches, except where a launch has about one block for each of the 152 SMs:
-    // blocks placed before the kernel ahead of them ends then share an SM while others have
-    // none (D2V16, 200 steps: 141x217 cells, 140 blocks, 4.72 ms plain, 4.97 programmatic;
-    // 200x200, 175 blocks, 5.75 / 5.12; 150x150, 95 blocks, 4.53 / 4.36)
     const unsigned blocks = grd.x * grd.y;
-    const bool early = blocks <= 96 || blocks > 152;
-    launch_after(early, k_pp32_collide<MODEL>, grd, blk, 0, st, P, S, do_msrc);
-    launch_after(early, k_pp32_faces1<MODEL>, grf, blk, 0, st, P, S);
+    // Two groups of threads where the blocks are few: each SM's share then takes the latency of
+    // one face instead of two.  One group on large grids, at the registers it runs best with
+    // (D2V16 three blocks an SM without spills, D2Q9 five).  us per step, two groups / one:
+    // D2V16 150x150 11.8 / 15.9, 330x330 (451 blocks) 26.0 / 26.9, 1024x1024 206 / 200;
+    // D2Q9 150x150 12.0 / 13.8, 330x330 22.1 / 25.3, 360x360 24.1 / 25.3, 400x400 28.6 / 27.0,
+    // 1024x1024 160 / 141 (four blocks 143, three 155).
+    if (blocks <= 3 * 152) launch_pdl(k_pp32_faces1<MODEL, 2, 2>, grd, dim3(32, 16), 0, st, P, S, do_msrc);
+    else launch_pdl(k_pp32_faces1<MODEL, 1, MODEL == PP16 ? 3 : 5>, grd, blk, 0, st, P, S, do_msrc);
     // face pass 2 compiled for three (D2Q9: four) resident blocks of 256 threads where the grid
     // fills them, with more registers for the few blocks of a small one (D2V16, us per step:
-    // 1024x1024 212 / 225, 400x400 35.6 / 38.2, 150x150 17.6 / 15.7; pass 1 for four / five)
-    if (blocks > 2 * 152) launch_after(early, k_pp32_faces2u<MODEL, MODEL == PP16 ? 3 : 4>, grd, blk, 0, st, P, S);
-    else launch_after(early, k_pp32_faces2u<MODEL, 2>, grd, blk, 0, st, P, S);
-    *launches += 3;
+    // with the passes of one more launch 1024x1024 212 / 225, 400x400 35.6 / 38.2, 150x150 17.6 / 15.7)
+    if (blocks > 2 * 152) launch_pdl(k_pp32_faces2u<MODEL, MODEL == PP16 ? 3 : 4>, grd, blk, 0, st, P, S);
+    else launch_pdl(k_pp32_faces2u<MODEL, 2>, grd, blk, 0, st, P, S);
+    *launches += 2;
     return cudaGetLastError();
 }
 
