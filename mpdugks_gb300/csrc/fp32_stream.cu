@@ -70,14 +70,18 @@ static int g_stream_nsm = 0, g_stream_blocks = 0;
 // the last, partly filled round is a large share of the step (measured: 2048^2 in 32-row
 // segments, 1.3 rounds, takes 1.28x the time of the best length), and the length is
 // searched instead: the fill of the last round, (items / warps) / ceil(items / warps),
-// times the share of a segment that is not warm-up, len / (len + 4), is maximised.
+// times the share of a segment that is not warm-up, len / (len + 4), is maximised, from
+// SEG_MIN rows up: a grid that fills less than one round is done when its longest segment is
+// (from 16 rows up, us a step of HCZ drops: 740x740 60.0 / 47.7, 680x680 in tiles 48.2 / 39.8,
+// 512x512 in tiles 30.1 / 26.4).
+constexpr int SEG_MIN = 5;
 int stream_segment_rows(int nstrips, int ny, int warps) {
     int seg = SEG_MAX;
     while (seg > 32 && (long long)nstrips * ((ny + seg - 1) / seg) < 4LL * warps) seg /= 2;
     if ((double)nstrips * ((ny + seg - 1) / seg) >= 8.0 * warps) return seg;
     int best = seg;
     double best_eff = -1.0;
-    for (int len = 16; len <= ny; ++len) {
+    for (int len = SEG_MIN; len <= ny; ++len) {
         const int n = (ny + len - 1) / len;
         const double waves = (double)nstrips * n / warps;
         const double eff = waves / std::ceil(waves) * ((double)ny / n / ((double)ny / n + 4.0));
@@ -116,22 +120,24 @@ static cudaError_t launch_stream_t(const P32 &P, const S32 &S, int first, int gi
         if ((e = cudaDeviceGetAttribute(&g_stream_nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
         ready = true;
     }
-    // the longest segment that still gives every resident warp about 4 segments
-    // (a long segment costs fewer warm-up rows, a short one less idle tail)
     const int nstrips = (P.nx + SW - 1) / SW, warps = g_stream_nsm * g_stream_blocks * WPB;
-    // a grid with fewer 32-row strip segments than a third of the resident warps leaves
-    // most of the GPU idle in this form: the tile kernel (same arithmetic, same results)
-    // runs it.  Measured (Rayleigh-Taylor, G cell-updates/s, streaming / tile): 256x1024
-    // 5.1 / 7.5 (320 segments), 768^2 9.2 / 8.5 (672), 512x2048 11.9 / 8.5 (1216), 1024^2
-    // 12.5 / 8.8 (1184), against 1824 resident warps.  (A slab partition reads halo rows,
-    // which only this form does, and so do NEE walls: it always runs those.)
-    if (!NEE && !(P.halo_lo || P.halo_hi) && 3LL * nstrips * ((P.ny + 31) / 32) < warps) {
-        *fallback = true;
-        return cudaSuccess;
-    }
     const int seg = stream_segment_rows(nstrips, P.ny, warps);
     const int nsegs = (P.ny + seg - 1) / seg;
     const int items = nstrips * nsegs;
+    // The tile kernel (same arithmetic, same results) takes the grids that it does sooner: its
+    // rounds of 30x14-cell tiles over the SMs, 6.1 us each (HCZ; AC 4.8, walls 6.7), against
+    // this kernel's rounds of segments, 2.7 us for each row and warm-up row (AC 2.1, walls 2.8).
+    // us a step, streaming / tile, HCZ: 300x300 17.9 / 13.1, 400x400 20.5 / 18.8, 450x450 23.3 /
+    // 24.4, 3000x64 23.1 / 22.4, 64x3000 22.9 / 29.3, 600x600 32.6 / 36.1, 700x700 40.3 / 49.2.
+    // (A slab partition reads halo rows, which only this form does, and so do NEE walls: it
+    // always runs those.)
+    const long long tiles = (long long)((P.nx + 29) / 30) * ((P.ny + 13) / 14);
+    const long long tile_rounds = (tiles + g_stream_nsm - 1) / g_stream_nsm;
+    const long long rounds = (items + warps - 1) / warps;
+    if (!NEE && !(P.halo_lo || P.halo_hi) && 4 * (min(seg, P.ny) + 4) * rounds > 9 * tile_rounds) {
+        *fallback = true;
+        return cudaSuccess;
+    }
     const int blocks = min((items + WPB - 1) / WPB, g_stream_nsm * g_stream_blocks);
     if (tmap) {
         launch_pdl(k_stream32<MODEL, WALLS, true, NEE>, blocks, WPB * 32, STREAM_SMEM, st, P, S, first, gin, gout, step,
