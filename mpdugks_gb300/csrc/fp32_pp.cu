@@ -195,8 +195,8 @@ __device__ __forceinline__ void pp_face2_at(const PPP &P, const PPS &S, int i, i
 
 // Face pass 2 and the update (Ark/Cpp/DUGKS2DSolver.cpp:748-792) with the cell macros
 // (Ark/Lib/D2Q9PP.cpp:89-109) in one launch: a block of 32x8 threads owns a 32x8-cell tile;
-// each thread computes the fluxes of its cell's west and south faces into shared memory,
-// 40 threads those of the tile's east column and north row (the next tiles' own faces,
+// each thread computes the fluxes of its cell's west and south faces into shared memory (by two
+// groups of 256 threads: the first the west faces, the second the south faces), 40 threads those of the tile's east column and north row (the next tiles' own faces,
 // whose forces those tiles store), and after a block barrier each thread updates its cell
 // from the four faces' fluxes, which never reach DRAM:
 //   rho_new = rho + drho, drho = dt/V sum_q (net face flux of q),
@@ -205,41 +205,45 @@ __device__ __forceinline__ void pp_face2_at(const PPP &P, const PPS &S, int i, i
 // px = dt/V (rho_W - rho_E)/2, py = dt/V (rho_S - rho_N)/2 (the e_q avg(rho) flux
 // divergence on unit cells, from the FP64 density); U, V, p, psi from float-float
 // sums, rho in FP64.
-template <int MODEL, int MIN_BLOCKS>
-__global__ void __launch_bounds__(256, MIN_BLOCKS) k_pp32_faces2u(PPP P, PPS S) {
+template <int MODEL, int GROUPS, int MIN_BLOCKS>
+__global__ void __launch_bounds__(256 * GROUPS, MIN_BLOCKS) k_pp32_faces2u(PPP P, PPS S) {
     pdl_wait();
     constexpr int Q = PPQ<MODEL>::Q;
     __shared__ float xs[Q][8][33];  // x-face fluxes of the tile's rows, columns 0 .. 32
     __shared__ float ys[Q][9][32];  // y-face fluxes of the tile's columns, rows 0 .. 8
-    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * 32 + tx;
+    const int tx = threadIdx.x, ty = threadIdx.y & 7, t = ty * 32 + tx;
+    const bool first = threadIdx.y < 8, do_x = GROUPS == 1 || first, do_y = GROUPS == 1 || !first;
     const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 8;
     const int w = min(32, P.nx - x0), h = min(8, P.ny - y0);
     const int i = x0 + tx, j = y0 + ty;
     const bool in = tx < w && ty < h;
     float out[Q];
-    if (in) {
+    if (in && do_x) {
         pp_face2_at<MODEL, true>(P, S, i, j, true, out);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (lat_u<MODEL>(q) != 0) xs[q][ty][tx] = out[q];
+    }
+    if (in && do_y) {
         pp_face2_at<MODEL, false>(P, S, i, j, true, out);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (lat_v<MODEL>(q) != 0) ys[q][ty][tx] = out[q];
     }
-    if (t < h) {  // x faces east of the tile (column x0 + w, periodic)
+    const int ne = GROUPS == 1 ? 32 : 0;  // first thread of the north row's faces
+    if (do_x && t < h) {  // x faces east of the tile (column x0 + w, periodic)
         pp_face2_at<MODEL, true>(P, S, wrapi(x0 + w, P.nx), y0 + t, false, out);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
             if (lat_u<MODEL>(q) != 0) xs[q][t][w] = out[q];
-    } else if (t >= 32 && t < 32 + w) {  // y faces north of the tile (row y0 + h, periodic)
-        pp_face2_at<MODEL, false>(P, S, x0 + t - 32, wrapi(y0 + h, P.ny), false, out);
+    } else if (do_y && t >= ne && t < ne + w) {  // y faces north of the tile (row y0 + h, periodic)
+        pp_face2_at<MODEL, false>(P, S, x0 + t - ne, wrapi(y0 + h, P.ny), false, out);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
-            if (lat_v<MODEL>(q) != 0) ys[q][h][t - 32] = out[q];
+            if (lat_v<MODEL>(q) != 0) ys[q][h][t - ne] = out[q];
     }
     __syncthreads();
-    if (!in) return;
+    if (!in || !first) return;
     const int pitch = P.pitch;
     const int ip = wrapi(i + 1, P.nx), im = wrapi(i - 1, P.nx), jn = wrapi(j + 1, P.ny), js = wrapi(j - 1, P.ny);
     const size_t c = (size_t)j * pitch + i;
@@ -321,8 +325,15 @@ static cudaError_t launch_pp_t(const PPP &P, const PPS &S, int do_msrc, cudaStre
     // face pass 2 compiled for three (D2Q9: four) resident blocks of 256 threads where the grid
     // fills them, with more registers for the few blocks of a small one (D2V16, us per step:
     // with the passes of one more launch 1024x1024 212 / 225, 400x400 35.6 / 38.2, 150x150 17.6 / 15.7)
-    if (blocks > 2 * 152) launch_pdl(k_pp32_faces2u<MODEL, MODEL == PP16 ? 3 : 4>, grd, blk, 0, st, P, S);
-    else launch_pdl(k_pp32_faces2u<MODEL, 2>, grd, blk, 0, st, P, S);
+    // Two groups for it too, on D2Q9 grids of one round of such blocks, two an SM (one group /
+    // two: 150x150 11.8 / 10.2, 256x256 16.6 / 14.8, 300x300 21.4 / 21.5), and for D2V16, whose
+    // threads need the registers of a whole SM then, where every block has one even when placed
+    // ahead of the launch before (128x128 12.1 / 11.4, 141x141, 90 blocks, 12.3 / 15.0).
+    const dim3 blk2(32, 16);
+    if (MODEL == PP16 ? blocks <= 76 : blocks <= 2 * 152)
+        launch_pdl(k_pp32_faces2u<MODEL, 2, MODEL == PP16 ? 1 : 2>, grd, blk2, 0, st, P, S);
+    else if (MODEL == PP16 && blocks <= 2 * 152) launch_pdl(k_pp32_faces2u<PP16, 1, 2>, grd, blk, 0, st, P, S);
+    else launch_pdl(k_pp32_faces2u<MODEL, 1, MODEL == PP16 ? 3 : 4>, grd, blk, 0, st, P, S);
     *launches += 2;
     return cudaGetLastError();
 }

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize('model,kw', [('PP9', {}), ('PP16', dict(d2v16_c=0.5))])
-@pytest.mark.parametrize('nx,ny', [(32, 8), (63, 9), (65, 1216), (33, 1825), (449, 257)])  # up to 456 / more tiles
+@pytest.mark.parametrize('nx,ny', [(32, 8), (63, 9), (200, 161), (65, 1216), (33, 1825), (449, 257)])  # 1 .. 510 tiles
 def test_tiles_equal_the_single_pass(model, kw, nx, ny, monkeypatch):
     out = []
     for passes in ('1', '3'):
