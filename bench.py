@@ -117,9 +117,10 @@ def fp64_pipe(lups: float) -> dict:
 # FP64 operations per cell-update of the plain FP64 step (k_collide + k_faces_ac + k_update
 # on the 512x2048 Rayleigh-Taylor case, reference-exact variant): ncu counts of the DADD,
 # DMUL and DFMA thread instructions of one step divided by the cells, a DFMA counted as two
-# (profiles/fp64_step_rt512x2048_fp64_ops.md)
-FP64_FLOPS_PER_CELL = 1720
-FP64_INSTR_PER_CELL = 1620
+# (profiles/fp64_step_rt512x2048_fp64_ops.md).  The products that the collision and the
+# faces form on the integer pipe are not in them.
+FP64_FLOPS_PER_CELL = 1174
+FP64_INSTR_PER_CELL = 963
 
 
 class ClockSampler:
@@ -535,7 +536,7 @@ def pseudopotential_bench(steps: int = 100) -> dict:
     for arm in ('fp32dev', 'fp32dev_single_pass', 'fp64', 'fp64fma'):
         from mpdugks_gb300 import capi
         prec = 'fp32dev' if arm.startswith('fp32') else arm
-        # the FP32 handle takes the three-pass step; the single-pass form beside it
+        # the FP32 handle takes the step of two tiled kernels; the single-pass form beside it
         if arm == 'fp32dev_single_pass':
             os.environ['DUGKS_PP_PASSES'] = '1'
         g = capi.GpuCase(c3_case(prec), n, n, False)

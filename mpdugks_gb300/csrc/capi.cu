@@ -143,7 +143,7 @@ struct dugks_handle {
     int init_kind = -1;       // the last dugks_gpu_init's kind and drop radius (drop L2 norm)
     double init_radius = 0.0;
     const double *pp_rho0 = nullptr;  // the density plane the step reads as created (checkpoint orientation)
-    bool pp_stream = false;           // FP32 pseudopotential: the single-pass step (else three passes)
+    bool pp_stream = false;           // FP32 pseudopotential: the single-pass step (else two launches)
 };
 
 static std::string g_create_err;
@@ -288,9 +288,9 @@ static bool d2v16_matrix_has_pair_form(const double (&iM)[16][16]) {
 static int create_pp32(dugks_handle *h, dugks_handle_t **out) {
     Params &P = h->P;
     h->pp32 = true;
-    // the three-pass step; DUGKS_PP_PASSES=1 in the environment selects the single-pass
+    // the step of two launches; DUGKS_PP_PASSES=1 in the environment selects the single-pass
     // streaming step (grids of at least 32 columns and 8 rows).  The two give the same
-    // results; on the GB300 the three-pass form is 1.75x faster (the single pass holds a row
+    // results; on the GB300 the two launches are 1.54x faster (the single pass holds a row
     // pipeline of 16 distributions per lane: ~10 warps per SM, latency-bound)
     const char *passes = std::getenv("DUGKS_PP_PASSES");
     h->pp_stream = P.nx >= 32 && P.ny >= 8 && passes && std::atoi(passes) == 1;

@@ -22,15 +22,14 @@
 // from one copy and written to the other (a segment reads rows its neighbours write).
 // Periodic in x and y (the pseudopotential models have no walls).
 //
-// Measured on the GB300 (D2V16, 1024^2): 2.35 G cell-updates/s against 4.10 for the three
-// passes, with the same results bit for bit (the equilibrium by opposite-direction pairs,
-// which the two forms share, took both up from 1.86 and 3.72).  A lane holds the row pipeline of 16
+// Measured on the GB300 (D2V16, 1024^2): 3.43 G cell-updates/s against 5.28 for the two tiled
+// kernels, with the same results bit for bit.  A lane holds the row pipeline of 16
 // distributions (168 registers when compiled for 5 blocks of 2 warps per SM -- 1.69 G at
 // the 215 the compiler takes unbounded, 2.00 G at 128 with spills) and the face moments
 // and the equation of state are serial float-float chains, so the ~10 resident warps
-// cannot hide their latency; the three passes run 40-80 registers a thread at high
-// occupancy and, for all their ~0.9 KB of traffic per cell-update, stay ahead.  The handle
-// therefore takes the three-pass step; DUGKS_PP_PASSES=1 selects this one.
+// cannot hide their latency; the tiled kernels run 64-80 registers a thread at two to three
+// times the occupancy and, for all their ~0.7 KB of traffic per cell-update, stay ahead.  The
+// handle therefore takes those; DUGKS_PP_PASSES=1 selects this one.
 #include <cuda_runtime.h>
 
 #include <cstdint>

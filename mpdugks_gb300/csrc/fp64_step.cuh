@@ -49,8 +49,10 @@
 //    viscosity, so the factors they appear in are powers of two, or drop out;
 //  * the equilibria of opposite directions share every product whose factors differ in
 //    sign only.
-// Passes of steps and a read-back, before and after: 512x2048 Rayleigh-Taylor box (HCZ, walls)
-// 4.07 -> 3.19 ms a step; 256x256 D2V16 0.453 -> 0.308 ms; 128x128 AC drop 74 -> 54 us.  The FMA
+// Passes of steps and a read-back, before and after these rewritings alone: 512x2048
+// Rayleigh-Taylor box (HCZ, walls) 4.07 -> 3.19 ms a step; 256x256 D2V16 0.453 -> 0.308 ms;
+// 128x128 AC drop 74 -> 54 us.  With the launch forms and the integer-pipe products below
+// (fp64_imul.cuh) 2.17 ms, 0.275 ms and 43 us.  The FMA
 // variant keeps the form its results were published with (another contraction moves the
 // velocities of a nearly resting fluid by 1e-9): only what is exact in any contraction, the
 // face reconstruction and the split by face direction, is shared: 333x257 HCZ drop 271 ->

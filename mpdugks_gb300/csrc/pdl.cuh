@@ -5,8 +5,8 @@
 // overlap the end of the one before.  pdl_wait() comes first in a kernel: completion is
 // transitive (the kernel before has waited for its own predecessor).
 // Passes of steps, plain / programmatic launches: 128x128 HCZ FP32 storage 2.24 / 1.61 ms (200
-// steps), UW 512x512 7.71 / 6.97 (100), D2Q9PP 150x133 4.29 / 3.95 (200), 32x24 AC FP64 1.86 /
-// 1.69 (50).
+// steps), UW 512x512 in four launches a step 7.71 / 6.97 (100), D2Q9PP 150x133 in three 4.29 /
+// 3.95 (200), 32x24 AC FP64 1.86 / 1.69 (50).
 #pragma once
 #include <cuda_runtime.h>
 
