@@ -324,7 +324,8 @@ static cudaError_t launch_pp_t(const PPP &P, const PPS &S, int do_msrc, cudaStre
     else launch_pdl(k_pp32_faces1<MODEL, 1, MODEL == PP16 ? 3 : 5>, grd, blk, 0, st, P, S, do_msrc);
     // face pass 2 compiled for three (D2Q9: four) resident blocks of 256 threads where the grid
     // fills them, with more registers for the few blocks of a small one (D2V16, us per step:
-    // with the passes of one more launch 1024x1024 212 / 225, 400x400 35.6 / 38.2, 150x150 17.6 / 15.7)
+    // when the step had three launches, 1024x1024 212 / 225, 400x400 35.6 / 38.2, 150x150 17.6 /
+    // 15.7).
     // Two groups for it too, on D2Q9 grids of one round of such blocks, two an SM (one group /
     // two: 150x150 11.8 / 10.2, 256x256 16.6 / 14.8, 300x300 21.4 / 21.5), and for D2V16, whose
     // threads need the registers of a whole SM then, where every block has one even when placed

@@ -86,8 +86,8 @@ __device__ __forceinline__ void load_cell(const S32 &S, size_t c, float2 (&Pq)[9
 
 // Collision of every cell: f-bar-plus pairs (B), the increments B - T (INC), the
 // averaged-field inputs (A) and, HCZ, the MacroSource outputs the next step reads.
-template <int MODEL>
-__global__ void __launch_bounds__(UBX *UBY) k_uw32_collide(P32 P, S32 S, float *U, int first) {
+template <int MODEL, int MIN_BLOCKS>
+__global__ void __launch_bounds__(UBX *UBY, MIN_BLOCKS) k_uw32_collide(P32 P, S32 S, float *U, int first) {
     pdl_wait();
     Cells k;
     if (!cell_of(P, k)) return;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(UBX *UBY) k_uw32_collide(P32 P, S32 S, float *
 // one direction later (one barrier a direction).  Every face is formed once per tile, then the
 // tile's cells are updated.
 // As four launches with the gradients and the fluxes in scratch planes the step moved 1.2 KB a
-// cell; now 0.53 KB.  512x512 69.7 -> 41.7 us a step, 2000x2000 1174 -> 604, 64x64 21.6 -> 8.9
+// cell; now 0.53 KB.  512x512 69.7 -> 40.8 us a step, 2000x2000 1174 -> 588, 64x64 21.6 -> 9.4
 // (there the launches).  What bounds it now is the latency of the direction loop and of the
 // face arithmetic at 24 to 32 warps an SM; the bytes alone take 20.7 us at 512x512.
 // Tiles of 14 rows (16 x 32 threads, two blocks an SM) are as fast on large grids and slower
@@ -306,7 +306,11 @@ __global__ void __launch_bounds__(UFX *UFY, MINB) k_uw32_tile(P32 P, S32 S, cons
 template <int MODEL>
 static cudaError_t launch_uw32_t(const P32 &P, const S32 &S, float *U, int first, cudaStream_t st) {
     const dim3 blk(UBX, UBY), grd((P.nx + UBX - 1) / UBX, (P.ny + UBY - 1) / UBY);
-    launch_pdl(k_uw32_collide<MODEL>, grd, blk, 0, st, P, S, U, first);
+    // 64 registers (a few of HCZ's spilled) where four blocks an SM make fewer rounds, else the
+    // 78 that the compiler takes.  Whole step, us: 256x256 14.4 / 15.5 at 64, 384x384 24.2 / 23.5,
+    // 512x512 42.0 / 40.8, 2000x2000 613 / 588.
+    launch_pdl(grd.x * grd.y <= 3 * 152 ? k_uw32_collide<MODEL, 3> : k_uw32_collide<MODEL, 4>, grd, blk, 0, st, P, S, U,
+               first);
     constexpr int FY = 8;
     const int ntx = (P.nx + UTW - 1) / UTW, tiles = ntx * ((P.ny + FY - 3) / (FY - 2));
     // Four resident blocks an SM at 64 registers (a few spilled) or three at 80: three while
