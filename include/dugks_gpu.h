@@ -219,11 +219,12 @@ int dugks_gpu_destroy(dugks_handle_t *h);
  * macroscopic fields only, Ark/Cpp/Output.cpp:537-606, so a reference run
  * cannot restart).  dugks_gpu_checkpoint writes the handle's whole device state
  * (distributions, macroscopic and auxiliary fields, ping-pong orientation,
- * step counter and the constants an upload derives) into buf, which must hold
+ * step counter) into buf, which must hold
  * dugks_gpu_checkpoint_bytes(h) bytes; it synchronises the handle's stream.
  * dugks_gpu_restore loads such a buffer into a handle created with the same
  * case and grid (DUGKS_EINVAL otherwise); the handle then continues bit for bit
- * as the saved one would have. */
+ * as the saved one would have.  Files of earlier libraries of the same version number
+ * are restored too (a longer header; another amount of UW scratch). */
 int dugks_gpu_checkpoint_bytes(const dugks_handle_t *h, size_t *bytes);
 /* Steps done since the upload (after a restore: since the saved run's upload). */
 int dugks_gpu_step_count(const dugks_handle_t *h, int64_t *steps);

@@ -1374,6 +1374,10 @@ extern "C" int dugks_gpu_last_error(const dugks_handle_t *h, char *buf, size_t l
 extern "C" int64_t dugks_gpu_launch_count(const dugks_handle_t *h) { return h ? h->launches : 0; }
 
 // ---- checkpoint / restart
+// A header and the arena.  The header holds nothing that the handle derives from its case: a
+// file's header may be longer (earlier version 1 files carry the FP32 pseudopotential constants
+// after these members), the arena starts
+// after header_bytes.
 namespace {
 struct CkptHeader {
     char magic[8];
@@ -1384,9 +1388,14 @@ struct CkptHeader {
     uint64_t arena_bytes;
     int64_t steps;
     int32_t pending, gcur, first, pp_pending, orient, pad1;
-    f32::PPP ppc;
 };
 const char CKPT_MAGIC[8] = {'D', 'U', 'G', 'K', 'S', 'C', 'K', '3'};
+
+// The part of the arena that holds state: all but the UW step's scratch, its last planes, whose
+// number is the step's own affair.
+size_t state_bytes(const dugks_handle *h) {
+    return h->uw32 ? (size_t)(reinterpret_cast<const char *>(h->uw32) - h->arena) : h->arena_bytes;
+}
 
 // orientation of the fused path's ping-pong views: 0 as created, 1 swapped
 int fused_orient(const dugks_handle *h) {
@@ -1428,7 +1437,6 @@ extern "C" int dugks_gpu_checkpoint(dugks_handle_t *h, void *buf, size_t len) {
     hd.first = h->first;
     hd.pp_pending = h->pp_pending;
     hd.orient = fused_orient(h);
-    hd.ppc = h->PPc;
     std::memcpy(buf, &hd, sizeof hd);
     cudaError_t e = cudaMemcpy(static_cast<char *>(buf) + sizeof hd, h->arena, h->arena_bytes, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(h, e, "checkpoint copy");
@@ -1442,23 +1450,24 @@ extern "C" int dugks_gpu_restore(dugks_handle_t *h, const void *buf, size_t len)
     if (len < sizeof hd) return fail(h, DUGKS_EINVAL, "checkpoint buffer too small");
     std::memcpy(&hd, buf, sizeof hd);
     if (std::memcmp(hd.magic, CKPT_MAGIC, sizeof hd.magic) != 0 || hd.version != 1 ||
-        hd.header_bytes != sizeof(CkptHeader))
+        hd.header_bytes < sizeof(CkptHeader))
         return fail(h, DUGKS_EINVAL, "not a checkpoint of this library version");
+    const size_t state = state_bytes(h);
     if (std::memcmp(&hd.cs, &h->cs, sizeof hd.cs) != 0 || std::memcmp(&hd.grid, &h->grid, sizeof hd.grid) != 0 ||
-        hd.arena_bytes != h->arena_bytes)
+        (h->uw32 ? hd.arena_bytes < state : hd.arena_bytes != state))
         return fail(h, DUGKS_EINVAL, "checkpoint of a different case or grid");
-    if (len < sizeof hd + hd.arena_bytes) return fail(h, DUGKS_EINVAL, "truncated checkpoint");
+    if (len < hd.header_bytes || len - hd.header_bytes < hd.arena_bytes)
+        return fail(h, DUGKS_EINVAL, "truncated checkpoint");
     int rc = sync_last(h);
     if (rc) return rc;
     cudaError_t e =
-        cudaMemcpy(h->arena, static_cast<const char *>(buf) + sizeof hd, h->arena_bytes, cudaMemcpyHostToDevice);
+        cudaMemcpy(h->arena, static_cast<const char *>(buf) + hd.header_bytes, state, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(h, e, "restore copy");
     h->steps = hd.steps;
     h->pending = hd.pending;
     h->gcur = hd.gcur;
     h->first = hd.first;
     h->pp_pending = hd.pp_pending;
-    if (h->pp32) h->PPc = hd.ppc;
     if (fused_orient(h) != hd.orient) {
         if (h->pp32) {
             pp32_swap(h);
