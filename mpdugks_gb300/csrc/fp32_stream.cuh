@@ -202,7 +202,7 @@ __device__ __forceinline__ bool stream_item(const P32 &P, const S32 &S, int firs
     auto load_phi = [&](int j) -> T {
         if (j <= y1 + 1 && row_ok(j)) {
             const long long c = cell(j);
-            return mk2(__ldg(S.phi + c), __ldg(S.phi + S.qs + c));
+            return mk2(S.phi[c], S.phi[S.qs + c]);
         }
         if ((wlo && j == -1) || (whi && j == ny)) {
             const size_t gr = gphi_row(gin, j < 0 ? 0 : 1);
@@ -239,7 +239,7 @@ __device__ __forceinline__ bool stream_item(const P32 &P, const S32 &S, int firs
         if (MODEL != AC && !first && k + 2 >= y0 - 1 && row_ok(k + 2) && colL) {
             const long long c2 = cell(k + 2);
 #pragma unroll
-            for (int a = 0; a < A_N; ++a) a6n[a] = __ldg(S.aux + (size_t)a * S.qs + c2);
+            for (int a = 0; a < A_N; ++a) a6n[a] = S.aux[(size_t)a * S.qs + c2];
         }
         ph2 = ph_n;
         ph_n = load_phi(k + 3);
@@ -366,7 +366,7 @@ __device__ __forceinline__ bool stream_item(const P32 &P, const S32 &S, int firs
             const long long c = cell(k);
             float a6[A_N];
 #pragma unroll
-            for (int a = 0; a < A_N; ++a) a6[a] = (MODEL != AC && !first) ? __ldg(S.aux + (size_t)a * S.qs + c) : 0.f;
+            for (int a = 0; a < A_N; ++a) a6[a] = (MODEL != AC && !first) ? S.aux[(size_t)a * S.qs + c] : 0.f;
             const T ph[8] = {SE, SWv, ph1, ph_m, E, W, mE, ph_mw};
             T inc[9];
             float src[6], phi, U, V;

@@ -4,6 +4,11 @@
 // complete (its writes are then visible), so the launch and the block start-up of a kernel
 // overlap the end of the one before.  pdl_wait() comes first in a kernel: completion is
 // transitive (the kernel before has waited for its own predecessor).
+// What such a kernel reads of an earlier kernel's writes it reads by ordinary loads: those of the
+// read-only path (__ldg, const __restrict__ parameters) are for data that stays unwritten for
+// the whole life of a kernel, which here begins before the last writes, and may be moved ahead
+// of the wait.  (The streaming step's phi and aux by either kind of load: 81.3 us a step at
+// 512x2048, 639 at 3072x3072.)
 // Passes of steps, plain / programmatic launches: 128x128 HCZ FP32 storage 2.24 / 1.61 ms (200
 // steps), UW 512x512 in four launches a step 7.71 / 6.97 (100), D2Q9PP 150x133 in three 4.29 /
 // 3.95 (200), 32x24 AC FP64 1.86 / 1.69 (50).
