@@ -44,7 +44,7 @@ cudaError_t launch_step64f(const PR<double> &P, const SR<double> &S, int first, 
                            cudaStream_t st, int64_t *launches, uint32_t step);
 void launch_macros64f(const PR<double> &P, const SR<double> &S, double *rho, double *u, double *v, double *p,
                       double *phi, int opitch, cudaStream_t st, int64_t *launches);
-cudaError_t launch_stream32(const P32 &P, const S32 &S, int first, int gin, int gout, cudaStream_t st,
+cudaError_t launch_stream32(const P32 &P, const S32 &S, StreamPlan &plan, int first, int gin, int gout, cudaStream_t st,
                             int64_t *launches, uint32_t step, const void *tmap, int zin, int *err);
 cudaError_t stream_tensor_map(void *map_out, float *base, int nx, int ny, int pitch, size_t qs);
 cudaError_t launch_uw32(const P32 &P, const S32 &S, float *U, int first, cudaStream_t st, int64_t *launches);
@@ -132,6 +132,7 @@ struct dugks_handle {
     bool has_tmap = false;
     const float *tmap_base = nullptr;
     int *kerr = nullptr;
+    f32::StreamPlan stream_plan;
     float *uw32 = nullptr;    // scratch planes of the FP32 UW step (f32::UW_PLANES)
     bool macros_fresh = false;
     double *out3 = nullptr;   // tau, Fx, Fy for output (allocated on first request)
@@ -960,8 +961,8 @@ extern "C" int dugks_gpu_step(dugks_handle_t *h, int nsteps, void *stream) {
             else if (h->uw32)
                 e = f32::launch_uw32(h->P32, h->S32, h->uw32, h->first, st, &h->launches);
             else
-                e = f32::launch_stream32(h->P32, h->S32, h->first, h->gcur, h->gcur ^ 1, st, &h->launches, sn,
-                                         h->has_tmap ? &h->tmap : nullptr, h->S32.df == h->tmap_base ? 0 : f32::PL_N,
+                e = f32::launch_stream32(h->P32, h->S32, h->stream_plan, h->first, h->gcur, h->gcur ^ 1, st,
+                                         &h->launches, sn, h->has_tmap ? &h->tmap : nullptr, h->S32.df == h->tmap_base ? 0 : f32::PL_N,
                                          h->kerr);
             if (e != cudaSuccess) return cuda_fail(h, e, "fp32 step launch");
             if (h->fused64) f32::swap_io(h->S64f);

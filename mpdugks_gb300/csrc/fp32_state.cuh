@@ -67,6 +67,15 @@ constexpr int PL_F = 0, PL_G = 9, PL_PHI = 17, PL_AUX = 19, PL_N = PL_AUX + A_N;
 //   INC: the collision increments B - T, laid out as B.
 constexpr int UW_B = 0, UW_A = 18, UW_INC = 24, UW_PLANES = 42;
 
+// How the streaming step takes a grid, chosen at its first step (launch_stream32) and kept by the
+// owner of the state: the choice searches over the segment lengths on the host.  Searched in every
+// step it took the calling thread 7 us for 2048 rows and 10.6 for 3000 (one step of 64x3000 alone:
+// 42.0 us, chosen once 31.8; of 512x2048 98.8 and 91.4; enqueueing a step 12.1 and 1.5).
+struct StreamPlan {
+    int seg = 0;         // rows of a strip segment (0: not chosen yet)
+    bool tiles = false;  // the tile kernel finishes the grid sooner
+};
+
 template <typename R>
 struct SR {
     R *df, *dg, *phi, *aux;      // the copy a step reads: planes PL_F, PL_G, PL_PHI, PL_AUX

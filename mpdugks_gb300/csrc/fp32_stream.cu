@@ -108,8 +108,8 @@ static cudaError_t stream_prepare() {
 }
 
 template <int MODEL, bool WALLS, bool NEE>
-static cudaError_t launch_stream_t(const P32 &P, const S32 &S, int first, int gin, int gout, cudaStream_t st,
-                                   uint32_t step, const CUtensorMap *tmap, int zin, int *err, bool *fallback) {
+static cudaError_t launch_stream_t(const P32 &P, const S32 &S, StreamPlan &plan, int first, int gin, int gout,
+                                   cudaStream_t st, uint32_t step, const CUtensorMap *tmap, int zin, int *err) {
     static bool ready = false;
     if (!ready) {
         cudaError_t e = stream_prepare<MODEL, WALLS, false, NEE>();
@@ -121,7 +121,9 @@ static cudaError_t launch_stream_t(const P32 &P, const S32 &S, int first, int gi
         ready = true;
     }
     const int nstrips = (P.nx + SW - 1) / SW, warps = g_stream_nsm * g_stream_blocks * WPB;
-    const int seg = stream_segment_rows(nstrips, P.ny, warps);
+    const bool chosen = plan.seg > 0;
+    if (!chosen) plan.seg = stream_segment_rows(nstrips, P.ny, warps);
+    const int seg = plan.seg;
     const int nsegs = (P.ny + seg - 1) / seg;
     const int items = nstrips * nsegs;
     // The tile kernel (same arithmetic, same results) takes the grids that it does sooner: its
@@ -134,10 +136,9 @@ static cudaError_t launch_stream_t(const P32 &P, const S32 &S, int first, int gi
     const long long tiles = (long long)((P.nx + 29) / 30) * ((P.ny + 13) / 14);
     const long long tile_rounds = (tiles + g_stream_nsm - 1) / g_stream_nsm;
     const long long rounds = (items + warps - 1) / warps;
-    if (!NEE && !(P.halo_lo || P.halo_hi) && 4 * (min(seg, P.ny) + 4) * rounds > 9 * tile_rounds) {
-        *fallback = true;
-        return cudaSuccess;
-    }
+    if (!chosen)
+        plan.tiles = !NEE && !(P.halo_lo || P.halo_hi) && 4 * (min(seg, P.ny) + 4) * rounds > 9 * tile_rounds;
+    if (plan.tiles) return cudaSuccess;
     const int blocks = min((items + WPB - 1) / WPB, g_stream_nsm * g_stream_blocks);
     if (tmap) {
         launch_pdl(k_stream32<MODEL, WALLS, true, NEE>, blocks, WPB * 32, STREAM_SMEM, st, P, S, first, gin, gout, step,
@@ -157,37 +158,36 @@ cudaError_t launch_step32(const P32 &P, const S32 &S, int first, int gin, int go
 // tmap: null, or the handle's 3-D tensor map over its two state copies (stream_tensor_map);
 // zin: the first plane of the copy this step reads (0 or PL_N); err: the word a staged
 // load that did not complete sets
-cudaError_t launch_stream32(const P32 &P, const S32 &S, int first, int gin, int gout, cudaStream_t st,
+cudaError_t launch_stream32(const P32 &P, const S32 &S, StreamPlan &plan, int first, int gin, int gout, cudaStream_t st,
                             int64_t *launches, uint32_t step, const void *tmap, int zin, int *err) {
     // the row window of a segment wraps at most once: grids of fewer than 8 rows
     // run the tile kernel (same arithmetic, same results)
     if (P.ny < 8) return launch_step32(P, S, first, gin, gout, st, launches, step);
     const CUtensorMap *tm = static_cast<const CUtensorMap *>(tmap);
     cudaError_t e = cudaErrorInvalidValue;
-    bool fallback = false;
     // NEE walls run the streaming form (the tile kernel has bounce-back walls only)
     switch (P.model * 4 + (P.walls ? 2 : 0) + (P.walls && P.nee ? 1 : 0)) {
         case AC * 4 + 0:
-            e = launch_stream_t<AC, false, false>(P, S, first, gin, gout, st, step, tm, zin, err, &fallback);
+            e = launch_stream_t<AC, false, false>(P, S, plan, first, gin, gout, st, step, tm, zin, err);
             break;
         case AC * 4 + 2:
-            e = launch_stream_t<AC, true, false>(P, S, first, gin, gout, st, step, tm, zin, err, &fallback);
+            e = launch_stream_t<AC, true, false>(P, S, plan, first, gin, gout, st, step, tm, zin, err);
             break;
         case AC * 4 + 3:
-            e = launch_stream_t<AC, true, true>(P, S, first, gin, gout, st, step, tm, zin, err, &fallback);
+            e = launch_stream_t<AC, true, true>(P, S, plan, first, gin, gout, st, step, tm, zin, err);
             break;
         case HCZ * 4 + 0:
-            e = launch_stream_t<HCZ, false, false>(P, S, first, gin, gout, st, step, tm, zin, err, &fallback);
+            e = launch_stream_t<HCZ, false, false>(P, S, plan, first, gin, gout, st, step, tm, zin, err);
             break;
         case HCZ * 4 + 2:
-            e = launch_stream_t<HCZ, true, false>(P, S, first, gin, gout, st, step, tm, zin, err, &fallback);
+            e = launch_stream_t<HCZ, true, false>(P, S, plan, first, gin, gout, st, step, tm, zin, err);
             break;
         case HCZ * 4 + 3:
-            e = launch_stream_t<HCZ, true, true>(P, S, first, gin, gout, st, step, tm, zin, err, &fallback);
+            e = launch_stream_t<HCZ, true, true>(P, S, plan, first, gin, gout, st, step, tm, zin, err);
             break;
         default: break;
     }
-    if (e == cudaSuccess && fallback) return launch_step32(P, S, first, gin, gout, st, launches, step);
+    if (e == cudaSuccess && plan.tiles) return launch_step32(P, S, first, gin, gout, st, launches, step);
     if (e == cudaSuccess) *launches += 1;
     return e;
 }

@@ -39,7 +39,7 @@ void derive_fp32(const Params &P, f32::P32 *Q);
 double rest_f(const Params &P, int q);
 }  // namespace internal
 namespace f32 {
-cudaError_t launch_stream32(const P32 &P, const S32 &S, int first, int gin, int gout, cudaStream_t st,
+cudaError_t launch_stream32(const P32 &P, const S32 &S, StreamPlan &plan, int first, int gin, int gout, cudaStream_t st,
                             int64_t *launches, uint32_t step, const void *tmap, int zin, int *err);
 void launch_macros32(const P32 &P, const S32 &S, double *rho, double *u, double *v, double *p, double *phi,
                      int opitch, cudaStream_t st, int64_t *launches);
@@ -64,6 +64,7 @@ constexpr int RED_BLOCKS = 152;  // blocks of a partition's reduction
 struct Part {
     int device = 0, row0 = 0, nrows = 0, lo = -1, hi = -1;  // lo/hi: neighbour partition, -1 = wall
     f32::P32 P{};
+    f32::StreamPlan plan;
     f32::S32 S{};          // current orientation (ping-pong swapped after each step)
     float *arena = nullptr;
     double *fields = nullptr;  // rho u v p phi [5][nrows][pitch] (download)
@@ -327,8 +328,8 @@ extern "C" int dugks_slabs_step(dugks_slabs_t *s, int nsteps) {
         const uint32_t sn = (uint32_t)s->steps;
         for (auto &q : s->parts) {
             cudaSetDevice(q.device);
-            cudaError_t e = f32::launch_stream32(q.P, q.S, s->first, s->gcur, s->gcur ^ 1, q.st, &s->launches, sn,
-                                                 nullptr, 0, nullptr);
+            cudaError_t e = f32::launch_stream32(q.P, q.S, q.plan, s->first, s->gcur, s->gcur ^ 1, q.st, &s->launches,
+                                                 sn, nullptr, 0, nullptr);
             if (e != cudaSuccess) return cuda_fail(e, "partition step");
         }
         if (s->multi_device) {  // every partition's step is done before its rows are copied
