@@ -366,13 +366,13 @@ static int create_pp32(dugks_handle *h, dugks_handle_t **out) {
     C.hc2 = 2.f * C.hc;
     C.hDt2 = 0.5f * C.hDt;
     {
-        // in FP32, one from the other: where a cell's force and its pressure gradient nearly
-        // balance, the ratio of the source's and the relaxation's rounded factors decides what is left
+        // one from the other: where a cell's force and its pressure gradient nearly balance, the
+        // ratio of the source's and the relaxation's rounded factors decides what is left
         const float tau = C.Tau0, aBP = (2.f * tau - C.hDt) / (2.f * tau + C.dt);
         C.bBP = 1.f - aBP;
         C.cBP = tau * C.bBP;
-        C.ah = 2.f * tau / (2.f * tau + C.hDt);
-        C.ch = tau * (1.f - C.ah);
+        C.ah = (float)(2.0 * P.Tau0 / (2.0 * P.Tau0 + P.hDt));
+        C.ch = (float)(P.Tau0 * (1.0 - (double)C.ah));
     }
     C.inv_6_2dx = (float)(1.0 / (P._2dx * 6));
     C.inv_6_2dy = (float)(1.0 / (P._2dy * 6));
@@ -402,6 +402,17 @@ static int create_pp32(dugks_handle *h, dugks_handle_t **out) {
                               RT * (0.3125 * A.N - 0.375 * A.Pc - A.R / 2) - A.jc, A.N / 16 - A.Pc / 8,
                               A.N / 16 - A.R / 2};
         for (int j = 0; j < 25; ++j) C.k[j] = (float)k[j];
+        // the equilibrium's momentum, sum_q xi_q de_q = rho u, from the rounded coefficients of u:
+        // the axis ring's takes up what the rounding of the others leaves (3e-8, at every
+        // relaxation of a cell and of a face), as it enters no other moment of these but xi_x^3.
+        // With the face relaxation above, error of u against 64 bits before / now / with the
+        // inverse moment matrix in FP32 instead of polynomials: 1024x1024, 50 steps 4.87e-6 /
+        // 4.52e-6 / 4.53e-6; 64x96, 200 steps 1.40e-5 / 1.27e-5 / 1.29e-5.  (The FP32 form of the
+        // density's gradients, the quotients by one reciprocal and psi by a reciprocal root leave
+        // these figures as they are with FP64 products, divisions and roots.  The cell's factors
+        // rounded from FP64 too would give 3.6e-7 for D2V16, and 2.2e-6 for 7.7e-7 in D2Q9.)
+        const double c = P.c16;
+        C.k[4] = (float)((1.0 - 4 * c * C.k[9] - 4 * c * C.k[15] - 8 * c * C.k[22]) / (2 * c));
     }
     e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
