@@ -180,13 +180,14 @@ __device__ __forceinline__ double cs_pressure(const Params &P, double rho) {
     const double r2 = rho * rho, m = 1.0 - rho;  // R = 1
     return rho * P.T_CS * (1.0 + rho + r2 - r2 * rho) / (m * m * m) - P.aCS * rho * rho;
 }
-// G = sign(p - rho RT), psi = sqrt(2 (p - rho RT) / G): the quotient by +-1 is the absolute
-// value, by 0 not a number; the sign is read from the bits
+// G = (p > rho RT) - (p < rho RT), psi = sqrt(2 (p - rho RT) / G): the quotient by +-1 is the
+// absolute value, by 0 not a number; the sign is read from the bits, 0 also for a difference that
+// is not a number
 __device__ __forceinline__ void calc_psi(const Params &P, double rho, double p, double &scg, double &psi) {
     const double d = p - rho * P.RT;
     const int hi = __double2hiint(d);
-    const bool zero = is_zero(d);
-    scg = zero ? 0.0 : (hi < 0 ? -1.0 : 1.0);
+    const bool zero = is_zero(d), nan = (hi & 0x7fffffff) > 0x7ff00000;  // (a sum's NaN is quiet)
+    scg = zero || nan ? 0.0 : (hi < 0 ? -1.0 : 1.0);
     const double r = sqrt(2.0 * fabs(d));
     psi = zero ? __hiloint2double(0x7ff80000, 0) : r;
 }
