@@ -77,6 +77,7 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
     const double ah = tauh / (tauh + P.hDt2), bh_ = 1.0 - ah, ch = tauh * bh_;
     const double ahs = UW ? ah : 0.5 * ah, hah = UW ? P.h_ah : P.h_ah2;
     const double Sx = both(F_PHIX), Sy = both(F_PHIY), ssum = Sx + Sy, sdif = Sy - Sx;
+    const bool far = warp_any<IM>(far_tail(Phi) || (MODEL == HCZ && (far_tail(Sx) || far_tail(Sy))));
     double *outf = lo ? (XF ? S.xlo_f : S.ylo_f) : (XF ? S.xff : S.yff);
     double *outh = lo ? (XF ? S.xlo_h : S.ylo_h) : (XF ? S.xfh : S.yfh);
     const size_t qs = lo ? (XF ? (size_t)ny : (size_t)pitch) : (XF ? S.qs : S.qsy);
@@ -110,7 +111,8 @@ __device__ __forceinline__ void face_ac(const Params &P, const State &S, int i, 
             }
         };
         Mul<IM> mul;
-        pair(mul);
+        if (far) mul.bad = 1;
+        else pair(mul);
         if (IM && mul.bad) {  // an operand beyond the integer product's window
             Mul<false> fp;
             pair(fp);

@@ -142,7 +142,8 @@ __device__ __forceinline__ bool face_of_thread(const Params &P, bool walls, bool
 static bool early_launch(const Params &P) { return pad32((unsigned)P.nx * P.ny) <= 32u * 152u * 4u; }
 // 32 x 8 blocks: from 486 k cells, or from 230 k where the integer products run with them (us
 // per step, one-warp blocks without / 32 x 8 with: 400x400 412 / 429, 460x460 519 / 521, 500x500
-// 609 / 589, 600x600 875 / 802)
+// 609 / 589, 600x600 875 / 802; along drops of 1000 steps, with the far tail of far_tail(): HCZ 480x480 564 /
+// 496-535, 600x600 876 / 781-828, AC 480x480 349 / 322-345, 600x600 540 / 510-546)
 static bool im_model(const Params &P) { return DUGKS_EXACT && (P.model == AC || P.model == HCZ) && !P.uw; }
 static bool wide_blocks(const Params &P) {
     const unsigned nx = P.nx;
@@ -151,7 +152,8 @@ static bool wide_blocks(const Params &P) {
 }
 // Products of the collision and the faces by the integer pipe (fp64_imul.cuh): the exact
 // variant on grids large enough for 32 x 8 blocks.  A face's 359 FP64 instructions become 277,
-// the collision's 373 become 250, and both kernels stay at 70-81 % of the pipe's issue rate.
+// the collision's 373 become 250, and both kernels stay at 70-81 % of the pipe's issue rate (a
+// pair's two forms in one body: the HCZ face kernel spills 200 bytes a thread at its 128 registers).
 // The code is four times as long, and the one-warp blocks of a smaller grid do not run through
 // it together.  us per step, without / with: 256x256 174 / 170, 400x400 412 / 430, 1000x1000
 // 2437 / 2059.  (Taken out again: the quotients' and moments' products too, which spilled, and
