@@ -964,7 +964,7 @@ extern "C" int dugks_gpu_step(dugks_handle_t *h, int nsteps, void *stream) {
     if (h->fp32) {
         for (int s = 0; s < nsteps; ++s) {
             const uint32_t sn = (uint32_t)(h->steps + s);
-            // FP32 storage: the streaming kernel (UW: the four-launch upwind step); the FP64
+            // FP32 storage: the streaming kernel (UW: the upwind step of two launches); the FP64
             // instance of the fused step: the tile kernel
             cudaError_t e;
             if (h->fused64)

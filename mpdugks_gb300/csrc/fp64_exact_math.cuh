@@ -52,8 +52,7 @@ __device__ __forceinline__ Xi4 xi4(double a, double b, double RT, double invRT) 
 
 // ---------------------------------------------------------------------------
 // D2V16 equilibrium: Macro16 (Ark/Lib/D2V16.cpp:125-145) at T = T0, p = rho R0 T0,
-// then the inverse moment matrix (Ark/Lib/D2V16.cpp:34-52): row by row in the exact variant,
-// by the parts even and odd in xi_x and xi_y in the FMA variant.
+// then the inverse moment matrix (Ark/Lib/D2V16.cpp:34-52), row by row.
 __device__ __forceinline__ void d2v16_eq(const Params &P, double rho, double u, double v, double *eq) {
     const double degrees = 3.0, degPlus2 = degrees + 2.0;
     const double T = P.T0, p = rho * P.R0 * T;
@@ -170,10 +169,9 @@ __device__ __forceinline__ void pp_eq(const Params &P, double rho, double U, dou
     else d2q9pp_eq(P, rho, U, V, eq);
 }
 
-// The He-Shan-Doolen projections (xi_q - u).F.  Exact variant: the reference's
-// fx (xi_u - U) + fy (xi_v - V), whose products are those of the model's few distinct velocity
-// components (D2Q9: -1, 0, 1; D2V16: c times -2 .. 2).  FMA variant: by opposite pairs, d - w
-// and -d - w with d = xi_q.F, w = u.F; a rest direction has -w.
+// The He-Shan-Doolen projections (xi_q - u).F: the reference's fx (xi_u - U) + fy (xi_v - V),
+// whose products are those of the model's few distinct velocity components (D2Q9: -1, 0, 1;
+// D2V16: c times -2 .. 2).
 template <int MODEL>
 __device__ __forceinline__ void pp_src_proj(const Params &P, double fx, double fy, double U, double V, double *pr) {
     constexpr int Q = MODEL == PP16 ? 16 : 9;

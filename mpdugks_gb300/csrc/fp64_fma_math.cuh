@@ -26,9 +26,8 @@ __device__ __forceinline__ Xi4 xi4(double a, double b, double RT, double invRT) 
 
 // ---------------------------------------------------------------------------
 // D2V16 equilibrium: Macro16 (Ark/Lib/D2V16.cpp:125-145) at T = T0, p = rho R0 T0,
-// then the inverse moment matrix: row by row in the exact variant, by opposite pairs in
-// the FMA variant, both without the structural zeros (the handle checks the matrix's form
-// when it is made).
+// then the inverse moment matrix by opposite pairs, without the structural zeros (the handle
+// checks the matrix's form when it is made).
 __device__ __forceinline__ void d2v16_eq(const Params &P, double rho, double u, double v, double *eq) {
     const double degrees = 3.0, degPlus2 = degrees + 2.0;
     const double T = P.T0, p = rho * P.R0 * T;
@@ -87,9 +86,8 @@ __device__ __forceinline__ void pp_eq(const Params &P, double rho, double U, dou
     else d2q9pp_eq(P, rho, U, V, eq);
 }
 
-// FMA variant: the He-Shan-Doolen projections (xi_q - u).F by opposite pairs, d - w and
-// -d - w with d = xi_q.F, w = u.F (xi_q' = -xi_q); a rest direction has -w.  The exact
-// variant keeps the reference's fx (xi_u - U) + fy (xi_v - V).
+// The He-Shan-Doolen projections (xi_q - u).F by opposite pairs, d - w and -d - w with
+// d = xi_q.F, w = u.F (xi_q' = -xi_q); a rest direction has -w.
 template <int MODEL>
 __device__ __forceinline__ void pp_src_proj(const Params &P, double fx, double fy, double U, double V, double *pr) {
     constexpr int Q = MODEL == PP16 ? 16 : 9;

@@ -11,10 +11,14 @@
 // face force) -- the Jacobi semantics of the face psi gradient.
 //
 // This file is compiled twice (see fp64_exact.cu / fp64_fast.cu):
-//  * DUGKS_EXACT = 1 with -fmad=false: every expression keeps the reference's
-//    operand association, divisions stay divisions and nothing is contracted
-//    into FMA, so the step reproduces the reference solver bit for bit (CUDA's
-//    FP64 +, -, *, / and sqrt are correctly rounded, like the host's);
+//  * DUGKS_EXACT = 1 with -fmad=false: every operation of the reference that rounds is
+//    rounded here alike, so the step gives the same doubles as the reference solver.
+//    The compiler contracts nothing; what is rewritten is what leaves the rounded values
+//    as they are: quotients by a shared divisor (qdiv_rn), powers of two taken into a
+//    fused multiply-add or a constant, terms that are zero, signs, products formed on the
+//    integer pipe (fp64_imul.cuh).  The one exception are subnormal numbers (a phase
+//    field below 1e-300 at the tip of its spreading tail): there a factor 1/2 does not
+//    commute with the rounding, and results may differ by some units of 2^-1074;
 //  * DUGKS_EXACT = 0 with FMA contraction and reciprocal multiplies: the same
 //    algorithm with fewer FP64 instructions, equal to the reference to rounding.
 #pragma once
@@ -28,14 +32,12 @@
 #endif
 #if DUGKS_EXACT
 #define DUGKS_KNS exact
-#define RDIV(x, d, invd) ((x) / (d))   // reference: a true division
 // x / d with invd = RN(1/d), the reciprocal of a divisor shared by several quotients:
 // correctly rounded (qdiv_rn), so the same double as the reference's division
 #define QDIV(x, d, invd) qdiv_rn((x), (d), (invd))
 #else
 #define DUGKS_KNS fast
-#define RDIV(x, d, invd) ((x) * (invd)) // one reciprocal, then multiplies
-#define QDIV(x, d, invd) ((x) * (invd))
+#define QDIV(x, d, invd) ((x) * (invd))  // one reciprocal, then multiplies
 #endif
 
 // The FP64 pipe bounds every kernel here (one warp instruction per 76 cycles and SM
